@@ -180,11 +180,13 @@ int egx_op_prepare(egx_ctx *ctx, egx_green *g, const double *zeta, const double 
 int egx_op_apply(egx_ctx *ctx, const double *x, double *y, int nrhs, int where);
 /* Same in complex64 (interleaved floats) with the complex64 tensor. */
 int egx_op_apply_c64(egx_ctx *ctx, const float *x, float *y, int nrhs, int where);
-/* The complex128 apply with its block contraction in double-FP32
- * arithmetic (Dot2 on float pairs, ~47 significant bits, no complex128 FMA):
- * the apply the mixed form uses for its refinement residuals. Same
- * arguments as egx_op_apply; nz <= 53 and 4 nrhs 3 nz float4 of staged
- * vectors <= 96 KiB, else the complex128 contraction runs. */
+/* The apply the mixed form uses for its refinement residuals: a complex128
+ * apply whose block contraction needs no complex128 FMA. For nz <= 48 it is
+ * egx_op_apply's own (error-free digit products); beyond, or without the
+ * memory for the digit copy, double-FP32 arithmetic (Dot2 on float pairs,
+ * ~47 significant bits) for nz <= 53 and 4 nrhs 3 nz float4 of staged
+ * vectors <= 96 KiB, else the complex128 contraction. Same arguments as
+ * egx_op_apply. */
 int egx_op_apply_ds(egx_ctx *ctx, const double *x, double *y, int nrhs, int where);
 
 /* ---- FFT (FftWrap plan_many_dft rank 2) -------------------------------- */

@@ -38,22 +38,12 @@ long nvec(const egx_ctx *ctx) { return (long)ctx->nx * ctx->ny * 3 * ctx->nz; }
 
 namespace {
 
-template <typename T>
-void upload_twiddles(DevBuf &dst, int n, cudaStream_t s) {
-    std::vector<double> t = twiddles(n);
-    if (sizeof(T) == sizeof(double)) {
-        dst.ensure(t.size() * sizeof(double));
-        EGX_CUDA(cudaMemcpyAsync(dst.p, t.data(), t.size() * sizeof(double), cudaMemcpyHostToDevice, s));
-    } else {
-        std::vector<float> f(t.begin(), t.end());
-        dst.ensure(f.size() * sizeof(float));
-        EGX_CUDA(cudaMemcpyAsync(dst.p, f.data(), f.size() * sizeof(float), cudaMemcpyHostToDevice, s));
-        EGX_CUDA(cudaStreamSynchronize(s));
-        return;
-    }
+template <typename V>
+void upload_table(DevBuf &dst, const V &t, cudaStream_t s) {
+    dst.ensure(t.size() * sizeof(t[0]));
+    EGX_CUDA(cudaMemcpyAsync(dst.p, t.data(), t.size() * sizeof(t[0]), cudaMemcpyHostToDevice, s));
     EGX_CUDA(cudaStreamSynchronize(s));
 }
-
 
 // r = (zeta - zeta0)/(zeta + conj zeta0) (A) or sqrt(Re zeta0)/(zeta + conj zeta0)
 // (Chi0) (ConvolutionOperator.PrepareRFunction, ConvolutionOperator.cs:113-143).
@@ -293,10 +283,10 @@ void ensure_twiddles(egx_ctx *ctx, int n0, int n1) {
     if (ctx->tw_n0 == n0 && ctx->tw_n1 == n1) return;
     ctx->p0 = make_fft_plan(n0);
     ctx->p1 = make_fft_plan(n1);
-    upload_twiddles<double>(ctx->tw0_64, n0, ctx->stream);
-    upload_twiddles<double>(ctx->tw1_64, n1, ctx->stream);
-    upload_twiddles<float>(ctx->tw0_32, n0, ctx->stream);
-    upload_twiddles<float>(ctx->tw1_32, n1, ctx->stream);
+    upload_table(ctx->tw0_64, fft_table64(n0), ctx->stream);
+    upload_table(ctx->tw1_64, fft_table64(n1), ctx->stream);
+    upload_table(ctx->tw0_32, fft_table32(n0), ctx->stream);
+    upload_table(ctx->tw1_32, fft_table32(n1), ctx->stream);
     ctx->tw_n0 = n0;
     ctx->tw_n1 = n1;
 }
@@ -946,9 +936,16 @@ int egx_fft2d(egx_ctx *ctx, double *buf, int n0, int n1, int howmany, int sign, 
         EGX_CHECK(sign == -1 || sign == 1, EGX_ERR_INVALID, "sign must be -1 or +1");
         set_device(ctx);
         FftPlan p0 = make_fft_plan(n0), p1 = make_fft_plan(n1);
-        DevBuf t0, t1;
-        upload_twiddles<double>(t0, n0, ctx->stream);
-        upload_twiddles<double>(t1, n1, ctx->stream);
+        if (ctx->fft_n0 != n0) {
+            ctx->fft_n0 = 0;
+            upload_table(ctx->fft_t0, fft_table64(n0), ctx->stream);
+            ctx->fft_n0 = n0;
+        }
+        if (ctx->fft_n1 != n1) {
+            ctx->fft_n1 = 0;
+            upload_table(ctx->fft_t1, fft_table64(n1), ctx->stream);
+            ctx->fft_n1 = n1;
+        }
         long n = (long)n0 * n1 * howmany;
         double2 *dbuf;
         if (where == EGX_DEVICE) {
@@ -958,7 +955,7 @@ int egx_fft2d(egx_ctx *ctx, double *buf, int n0, int n1, int howmany, int sign, 
             dbuf = ctx->fftbuf.as<double2>();
             EGX_CUDA(cudaMemcpyAsync(dbuf, buf, n * sizeof(double2), cudaMemcpyHostToDevice, ctx->stream));
         }
-        fft2d<double>(dbuf, n0, n1, howmany, sign, t0.as<double2>(), t1.as<double2>(), p0, p1, ctx->stream,
+        fft2d<double>(dbuf, n0, n1, howmany, sign, ctx->fft_t0.as<double2>(), ctx->fft_t1.as<double2>(), p0, p1, ctx->stream,
                       &ctx->launches);
         if (where != EGX_DEVICE)
             EGX_CUDA(cudaMemcpyAsync(buf, dbuf, n * sizeof(double2), cudaMemcpyDeviceToHost, ctx->stream));

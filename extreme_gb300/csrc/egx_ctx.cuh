@@ -58,7 +58,8 @@ struct egx_ctx {
     int precond_kind = EGX_PRECOND_GMRES;
     egx_precond_fn precond_fn = nullptr;
     void *precond_user = nullptr;
-    egx::DevBuf fftbuf;
+    egx::DevBuf fftbuf, fft_t0, fft_t1;
+    int fft_n0 = 0, fft_n1 = 0;  // lengths of egx_fft2d's tables in fft_t0, fft_t1
     // egx_set_graphs: the inner GMRES cycle of the flexible preconditioner
     // captured as one CUDA graph (staging buffers, the executable graph and
     // the key of everything it bakes in)

@@ -11,14 +11,85 @@
 // 7-smooth length.
 #pragma once
 
+#include <algorithm>
+#include <cmath>
+
 #include "egx_common.cuh"
 
 namespace egx {
+
+// The generic transform's plan (egx_fft_gen.cuh).
+//
+// Stages of a transform of length n <= kGenMax. div: ceil(2^20 / Ns), the
+// quotient j / Ns of an item; off: the stage's first entry of the twiddle
+// table [jm][r - 1]; sh: the bits that its inputs give back (double).
+constexpr int kGenMax = 1024;
+struct GenPlan {
+    int n = 0, ns = 0;
+    int rows = 0;  // items of the first stage
+    int R[6], Ns[6], div[6], off[6], sh[6];
+    int sh_sum = 0;
+    int cls = 0;  // class of the largest kernel that a stage needs (EGX_RADIX_SWITCH)
+};
+
+// Host: few stages, the smallest radix last, the second smallest first (the
+// stages in the middle then have at most as many items as the first and can
+// work in place); ns = 0 when the length has no such plan.
+inline GenPlan make_gen_plan(int n) {
+    GenPlan p;
+    if (n < 4 || n > kGenMax) return p;
+    int best[6] = {}, nb = 7, cur[6] = {};
+    // radices in ascending order; fewest stages, then the more even ones (the
+    // larger smallest radix, the larger second smallest, ...)
+    auto search = [&](auto &&self, int left, int from, int depth) -> void {
+        if (left == 1) {
+            bool better = depth < nb;
+            for (int i = 0; depth == nb && i < depth; i++)
+                if (cur[i] != best[i]) {
+                    better = cur[i] > best[i];
+                    break;
+                }
+            if (depth >= 2 && better) {
+                nb = depth;
+                for (int i = 0; i < depth; i++) best[i] = cur[i];
+            }
+            return;
+        }
+        if (depth >= 6 || depth >= nb) return;
+        for (int r = from; r <= 10; r++)
+            if (left % r == 0) {
+                cur[depth] = r;
+                self(self, left / r, r, depth + 1);
+            }
+    };
+    search(search, n, 2, 0);
+    if (nb > 6) return p;
+    p.n = n;
+    p.ns = nb;
+    for (int s = 0; s < nb; s++) p.R[s] = s + 1 < nb ? best[s + 1] : best[0];
+    p.rows = n / p.R[0];
+    int ns = 1, off = 0;
+    double top = 59.5;  // log2 of a bound of the complex values (double: see egx_fft_gen.cuh)
+    for (int s = 0; s < nb; s++) {
+        p.Ns[s] = ns;
+        p.div[s] = ((1 << 20) + ns - 1) / ns;
+        p.off[s] = off;
+        top += std::log2((double)p.R[s]);
+        p.sh[s] = s ? std::max(2, (int)std::ceil(top - 62.85)) : 0;
+        top -= p.sh[s];
+        p.sh_sum += p.sh[s];
+        p.cls = std::max(p.cls, p.R[s] == 7 ? 3 : (p.R[s] > 8 ? 2 : ((p.R[s] & (p.R[s] - 1)) ? 1 : 0)));
+        if (s) off += ns * (p.R[s] - 1);
+        ns *= p.R[s];
+    }
+    return p;
+}
 
 struct FftPlan {
     int n;
     int nstages;
     int radix[16];
+    GenPlan gen;
 };
 
 // Host: radix sequence for n (prefers 8, then 4, 2, and 7, 6, 5, 3).
@@ -26,6 +97,7 @@ inline FftPlan make_fft_plan(int n) {
     FftPlan p;
     p.n = n;
     p.nstages = 0;
+    p.gen = make_gen_plan(n);
     int m = n;
     while (m > 1) {
         int r = 0;
@@ -205,6 +277,10 @@ __device__ C<T> *fft_smem(C<T> *a, C<T> *b, const FftPlan &plan, int bt, const C
 
 // Host-side twiddle table W_n^m = exp(-2*pi*i*m/n).
 std::vector<double> twiddles(int n);
+// The device tables of a length: n plain twiddles (the register and Stockham
+// kernels), then the stage table of the generic plan.
+std::vector<double> fft_table64(int n);
+std::vector<float> fft_table32(int n);
 
 // Columns per CTA so that the two shared buffers stay near 64 KB.
 inline int fft_cols(int n, size_t elem) {

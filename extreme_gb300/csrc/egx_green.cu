@@ -734,6 +734,20 @@ X *dev_upload(DevBuf &b, const std::vector<X> &v, cudaStream_t s) {
     return b.as<X>();
 }
 
+// the workspace's FFT tables of lengths n0 and n1, kept while they fit
+void fft_tables64(GreenWorkspace &w, int n0, int n1, cudaStream_t s) {
+    if (w.n64[0] == n0 && w.n64[1] == n1) return;
+    dev_upload(w.tw0, fft_table64(n0), s);
+    dev_upload(w.tw1, fft_table64(n1), s);
+    w.n64[0] = n0, w.n64[1] = n1;
+}
+void fft_tables32(GreenWorkspace &w, int n0, int n1, cudaStream_t s) {
+    if (w.n32[0] == n0 && w.n32[1] == n1) return;
+    dev_upload(w.tw0_32, fft_table32(n0), s);
+    dev_upload(w.tw1_32, fft_table32(n1), s);
+    w.n32[0] = n0, w.n32[1] = n1;
+}
+
 double ms_since(std::chrono::steady_clock::time_point t0) {
     return std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
 }
@@ -1246,13 +1260,8 @@ void build_green(const GreenModel &m, int n_hankels, cudaStream_t s, DevBuf &qua
     FftPlan p0 = make_fft_plan(2 * m.nx), p1 = make_fft_plan(2 * m.ny);
     DevBuf &tw0 = w.tw0, &tw1 = w.tw1;
     {
-        std::vector<double> t0 = twiddles(2 * m.nx), t1 = twiddles(2 * m.ny);
-        dev_upload(tw0, t0, s);
-        dev_upload(tw1, t1, s);
-        if (lateral_fft32) {
-            dev_upload(w.tw0_32, std::vector<float>(t0.begin(), t0.end()), s);
-            dev_upload(w.tw1_32, std::vector<float>(t1.begin(), t1.end()), s);
-        }
+        fft_tables64(w, 2 * m.nx, 2 * m.ny, s);
+        if (lateral_fft32) fft_tables32(w, 2 * m.nx, 2 * m.ny, s);
     }
     double *radii_dev = dev_upload(d_radii, radii, s);
 
@@ -1302,7 +1311,7 @@ void build_green(const GreenModel &m, int n_hankels, cudaStream_t s, DevBuf &qua
         d_IA.ensure((size_t)nu * nseg * ntrans * sizeof(double2));
         d_IB.ensure((size_t)nu * nseg * ntrans * sizeof(double2));
         // the mixed form's face sums run in double-FP32 on float pairs
-        const bool face_ds = lateral_fft32 && fft_lines_sym_ok(2 * m.nx) && fft_lines_sym_ok(2 * m.ny);
+        const bool face_ds = lateral_fft32 && fft_lines_sym_ok<float>(p0, 0) && fft_lines_sym_ok<float>(p1, 0);
         if (face_ds) {
             w.d_IA32.ensure((size_t)nu * nseg * ntrans * sizeof(float4));
             w.d_IB32.ensure((size_t)nu * nseg * ntrans * sizeof(float4));
@@ -1333,8 +1342,8 @@ void build_green(const GreenModel &m, int n_hankels, cudaStream_t s, DevBuf &qua
         // by the FFT's loads (half the y lines, a quarter of the memory);
         // otherwise the full 2nx x 2ny grid populated by mirroring
         const int n0 = 2 * m.nx, n1 = 2 * m.ny;
-        const bool compact = fft_lines_sym_ok(n0) && fft_lines_sym_ok(n1);
-        const bool fft32 = lateral_fft32 && compact;
+        const bool fft32 = face_ds;
+        const bool compact = fft32 || (fft_lines_sym_ok<double>(p0, m.ny + 1) && fft_lines_sym_ok<double>(p1, m.nx));
         const long cells4 = compact ? (long)(m.nx + 1) * (m.ny + 1) : 4L * m.nx * m.ny;
         const int row = compact ? m.ny + 1 : n1;
         int tc = (int)std::min<long>(blk, std::max<long>(1, (long)(1.5e9 / (cells4 * sizeof(double2)))));
@@ -1378,17 +1387,17 @@ void build_green(const GreenModel &m, int n_hankels, cudaStream_t s, DevBuf &qua
                 ev = tm ? tm->begin(EGX_K_GREEN_FFT, s) : -1;
                 if (fft32) {
                     // as below, in complex64
-                    fft_lines_sym<float>(w.d_buf32.as<float2>(), m.nx, (long)row * tcc, tcc, tcc, py[c], m.ny + 1, n1,
+                    fft_lines_sym<float>(w.d_buf32.as<float2>(), m.nx, (long)row * tcc, tcc, tcc, py[c], m.ny + 1, p1,
                                          w.tw1_32.as<float2>(), -1, s, launches);
                     fft_lines_sym<float>(w.d_buf32.as<float2>(), m.ny + 1, tcc, (long)row * tcc, tcc, px[c], m.nx + 1,
-                                         n0, w.tw0_32.as<float2>(), -1, s, launches);
+                                         p0, w.tw0_32.as<float2>(), -1, s, launches);
                 } else if (compact) {
                     // y along the nx computed rows, ky <= ny kept; then x along
                     // ky <= ny, kx <= nx kept (row nx of the input is zero)
-                    fft_lines_sym<double>(d_buf.as<double2>(), m.nx, (long)row * tcc, tcc, tcc, py[c], m.ny + 1, n1,
+                    fft_lines_sym<double>(d_buf.as<double2>(), m.nx, (long)row * tcc, tcc, tcc, py[c], m.ny + 1, p1,
                                           tw1.as<double2>(), -1, s, launches);
                     fft_lines_sym<double>(d_buf.as<double2>(), m.ny + 1, tcc, (long)row * tcc, tcc, px[c], m.nx + 1,
-                                          n0, tw0.as<double2>(), -1, s, launches);
+                                          p0, tw0.as<double2>(), -1, s, launches);
                 } else {
                     // y along all 2nx rows; x along ky <= ny, kx <= nx kept
                     fft_lines<double>(d_buf.as<double2>(), n0, (long)n1 * tcc, tcc, tcc, n1, n1, p1,
@@ -1581,14 +1590,8 @@ void build_level_green(const GreenModel &m, int n_hankels, double z, double shx,
     const int n0 = 2 * m.nx, n1 = 2 * m.ny;
     FftPlan p0 = make_fft_plan(n0), p1 = make_fft_plan(n1);
     {
-        std::vector<double> t0 = twiddles(n0), t1 = twiddles(n1);
-        if (fft32) {
-            dev_upload(w.tw0_32, std::vector<float>(t0.begin(), t0.end()), s);
-            dev_upload(w.tw1_32, std::vector<float>(t1.begin(), t1.end()), s);
-        } else {
-            dev_upload(w.tw0, t0, s);
-            dev_upload(w.tw1, t1, s);
-        }
+        if (fft32) fft_tables32(w, n0, n1, s);
+        else fft_tables64(w, n0, n1, s);
     }
     for (int c = 0; c < ncomp; c++) {
         const long n = ncell * m.nz;

@@ -124,7 +124,7 @@ __global__ void k_bwd_y(const C<T> *__restrict__ buf, const C<T> *__restrict__ x
 
 // ------------------------------------------------------------------
 // The same three steps on the register-resident DFT (egx_fft_reg.cuh) for
-// lengths in {64, 128, 256, 512}: one CTA per line and 128-byte tile of
+// complex64 lengths in {64, 128, 256, 512}: one CTA per line and 128-byte tile of
 // columns, every global access a whole row segment of BT columns. The y
 // passes and the forward x pass run 64-byte tiles (512 threads per CTA for
 // complex64, four CTAs per SM at 32 registers), whose CTAs overlap their
@@ -262,11 +262,14 @@ static void launch_reg_tile(int which, cudaStream_t s, int nlines, const C<T> *x
                                           sign);
 }
 
-// returns false when n has no register plan
+// complex64 lengths with a register plan (complex128 takes the generic
+// transform's integer arithmetic at every length); false when there is none
 template <typename T>
 static bool run_reg(int n, int which, int nlines, int B, cudaStream_t s, const C<T> *x, const OperatorData<T> *op,
                     C<T> *buf, C<T> *y, const OpDims *d, long lstride, long estride, int nload, int nstore,
                     const C<T> *tw, int sign, int tile = 0) {
+    if constexpr (std::is_same<T, double>::value) return false;
+    else {
     if (!reg_fft_ok(n)) return false;
     switch (n) {
         case 64: launch_reg_tile<T, 64>(which, s, nlines, x, op, buf, y, d, lstride, estride, B, nload, nstore, tw, sign, tile); break;
@@ -275,6 +278,7 @@ static bool run_reg(int n, int which, int nlines, int B, cudaStream_t s, const C
         default: launch_reg_tile<T, 512>(which, s, nlines, x, op, buf, y, d, lstride, estride, B, nload, nstore, tw, sign, tile); break;
     }
     return true;
+    }
 }
 
 // Block contraction, one CTA per stored quadrant point (a, b). The block is
@@ -494,11 +498,17 @@ void operator_apply(const OpDims &d, const OperatorData<T> &op, const C<T> *G, c
                     long *launches, Timers *tm, int *err) {
     const int n0 = 2 * d.nx, n1 = 2 * d.ny;
     const int koff = sizeof(T) == sizeof(double) ? 0 : EGX_K_C64;
+    // chi0 of the mixed form is a complex64 apply whose rounding (1e-7) is
+    // part of the system that the refinement then solves to any tolerance:
+    // it stays on the kernels that have always made it, so that a solve's
+    // result does not move by 1e-7 with the faster ones of the inner applies
+    const bool gen = std::is_same<T, double>::value || op.type != EGX_OP_CHI0;
     int ev;
     // 1. r*x, forward factors, zero padding, DFT along y (rows i < nx)
     {
         ev = tm ? tm->begin(EGX_K_FWD_Y + koff, s) : -1;
-        if (!run_reg<T>(n1, 0, d.nx, d.B, s, x, &op, buf, nullptr, &d, 0, 0, 0, 0, tw1, -1, d.fft_tile)) {
+        if (!run_reg<T>(n1, 0, d.nx, d.B, s, x, &op, buf, nullptr, &d, 0, 0, 0, 0, tw1, -1, d.fft_tile) &&
+            !(gen && gen_fwd_y<T>(p1, x, op, buf, d, tw1, s))) {
             int bt = fft_cols(n1, sizeof(C<T>));
             size_t sm = 2 * (size_t)n1 * bt * sizeof(C<T>);
             set_smem<T>((const void *)k_fwd_y<T>, sm);
@@ -511,7 +521,8 @@ void operator_apply(const OpDims &d, const OperatorData<T> &op, const C<T> *G, c
     {
         ev = tm ? tm->begin(EGX_K_FWD_X + koff, s) : -1;
         if (!run_reg<T>(n0, 1, n1, d.B, s, nullptr, nullptr, buf, nullptr, nullptr, d.B, (long)n1 * d.B, d.nx, n0,
-                        tw0, -1, d.fft_tile)) {
+                        tw0, -1, d.fft_tile) &&
+            !(gen && gen_lines<T>(p0, buf, n1, d.B, (long)n1 * d.B, d.B, d.nx, n0, tw0, -1, s))) {
             int bt = fft_cols(n0, sizeof(C<T>));
             size_t sm = 2 * (size_t)n0 * bt * sizeof(C<T>);
             set_smem<T>((const void *)k_lines<T>, sm);
@@ -560,7 +571,8 @@ void operator_apply(const OpDims &d, const OperatorData<T> &op, const C<T> *G, c
     {
         ev = tm ? tm->begin(EGX_K_BWD_X + koff, s) : -1;
         if (!run_reg<T>(n0, 1, n1, d.B, s, nullptr, nullptr, buf, nullptr, nullptr, d.B, (long)n1 * d.B, n0, d.nx,
-                        tw0, +1, d.fft_tile)) {
+                        tw0, +1, d.fft_tile) &&
+            !(gen && gen_lines<T>(p0, buf, n1, d.B, (long)n1 * d.B, d.B, n0, d.nx, tw0, +1, s))) {
             int bt = fft_cols(n0, sizeof(C<T>));
             size_t sm = 2 * (size_t)n0 * bt * sizeof(C<T>);
             set_smem<T>((const void *)k_lines<T>, sm);
@@ -573,7 +585,8 @@ void operator_apply(const OpDims &d, const OperatorData<T> &op, const C<T> *G, c
     // 5. inverse DFT along y, extraction, last step
     {
         ev = tm ? tm->begin(EGX_K_BWD_Y + koff, s) : -1;
-        if (!run_reg<T>(n1, 2, d.nx, d.B, s, x, &op, buf, y, &d, 0, 0, 0, 0, tw1, +1, d.fft_tile)) {
+        if (!run_reg<T>(n1, 2, d.nx, d.B, s, x, &op, buf, y, &d, 0, 0, 0, 0, tw1, +1, d.fft_tile) &&
+            !(gen && gen_bwd_y<T>(p1, buf, x, op, y, d, tw1, s))) {
             int bt = fft_cols(n1, sizeof(C<T>));
             size_t sm = 2 * (size_t)n1 * bt * sizeof(C<T>);
             set_smem<T>((const void *)k_bwd_y<T>, sm);
@@ -587,78 +600,63 @@ void operator_apply(const OpDims &d, const OperatorData<T> &op, const C<T> *G, c
 }
 
 template <typename T>
-void fft2d(C<T> *buf, int n0, int n1, int howmany, int sign, const C<T> *tw0, const C<T> *tw1, const FftPlan &p0,
-           const FftPlan &p1, cudaStream_t s, long *launches) {
-    if (!run_reg<T>(n1, 1, n0, howmany, s, nullptr, nullptr, buf, nullptr, nullptr, (long)n1 * howmany, howmany, n1,
-                    n1, tw1, sign)) {
-        int bt = fft_cols(n1, sizeof(C<T>));
-        size_t sm = 2 * (size_t)n1 * bt * sizeof(C<T>);
-        set_smem<T>((const void *)k_lines<T>, sm);
-        dim3 grid(n0, (howmany + bt - 1) / bt);
-        k_lines<T><<<grid, threads_for(n1 * bt / 2), sm, s>>>(buf, (long)n1 * howmany, howmany, howmany, n1, n1, p1,
-                                                              tw1, bt, sign);
-    }
-    if (!run_reg<T>(n0, 1, n1, howmany, s, nullptr, nullptr, buf, nullptr, nullptr, howmany, (long)n1 * howmany, n0,
-                    n0, tw0, sign)) {
-        int bt = fft_cols(n0, sizeof(C<T>));
-        size_t sm = 2 * (size_t)n0 * bt * sizeof(C<T>);
-        set_smem<T>((const void *)k_lines<T>, sm);
-        dim3 grid(n1, (howmany + bt - 1) / bt);
-        k_lines<T><<<grid, threads_for(n0 * bt / 2), sm, s>>>(buf, howmany, (long)n1 * howmany, howmany, n0, n0, p0,
-                                                              tw0, bt, sign);
-    }
-    EGX_CUDA(cudaGetLastError());
-    if (launches) *launches += 2;
-}
-
-template <typename T>
 void fft_lines(C<T> *buf, int nlines, long lstride, long estride, int B, int nload, int nstore, const FftPlan &p,
                const C<T> *tw, int sign, cudaStream_t s, long *launches) {
-    if (run_reg<T>(p.n, 1, nlines, B, s, nullptr, nullptr, buf, nullptr, nullptr, lstride, estride, nload, nstore, tw,
-                   sign)) {
-        EGX_CUDA(cudaGetLastError());
-        if (launches) *launches += 1;
-        return;
+    if (!run_reg<T>(p.n, 1, nlines, B, s, nullptr, nullptr, buf, nullptr, nullptr, lstride, estride, nload, nstore, tw,
+                    sign) &&
+        !gen_lines<T>(p, buf, nlines, lstride, estride, B, nload, nstore, tw, sign, s)) {
+        int bt = fft_cols(p.n, sizeof(C<T>));
+        size_t sm = 2 * (size_t)p.n * bt * sizeof(C<T>);
+        set_smem<T>((const void *)k_lines<T>, sm);
+        dim3 grid(nlines, (B + bt - 1) / bt);
+        k_lines<T><<<grid, threads_for(p.n * bt / 2), sm, s>>>(buf, lstride, estride, B, nload, nstore, p, tw, bt, sign);
     }
-    int bt = fft_cols(p.n, sizeof(C<T>));
-    size_t sm = 2 * (size_t)p.n * bt * sizeof(C<T>);
-    set_smem<T>((const void *)k_lines<T>, sm);
-    dim3 grid(nlines, (B + bt - 1) / bt);
-    k_lines<T><<<grid, threads_for(p.n * bt / 2), sm, s>>>(buf, lstride, estride, B, nload, nstore, p, tw, bt, sign);
     EGX_CUDA(cudaGetLastError());
     if (launches) *launches += 1;
 }
-
-template <typename T, int N>
-static void launch_sym(dim3 grid, cudaStream_t s, C<T> *buf, long lstride, long estride, int B, T par, int nstore,
-                       const C<T> *tw, int sign) {
-    reg_attr<T, N>((const void *)k_lines_sym_r<T, N>);
-    k_lines_sym_r<T, N><<<grid, reg_threads<N, T>(), reg_smem<N, T>(), s>>>(buf, lstride, estride, B, par, nstore, tw,
-                                                                            sign);
-}
-
-bool fft_lines_sym_ok(int n) { return reg_fft_ok(n); }
 
 template <typename T>
-void fft_lines_sym(C<T> *buf, int nlines, long lstride, long estride, int B, int parity, int nstore, int n,
-                   const C<T> *tw, int sign, cudaStream_t s, long *launches) {
-    EGX_CHECK(reg_fft_ok(n), EGX_ERR_INVALID, "mirrored FFT lines need a length in {64, 128, 256, 512}");
-    dim3 grid(nlines, (B + RegCols<T>::BT - 1) / RegCols<T>::BT);
-    const T par = (T)parity;
-    switch (n) {
-        case 64: launch_sym<T, 64>(grid, s, buf, lstride, estride, B, par, nstore, tw, sign); break;
-        case 128: launch_sym<T, 128>(grid, s, buf, lstride, estride, B, par, nstore, tw, sign); break;
-        case 256: launch_sym<T, 256>(grid, s, buf, lstride, estride, B, par, nstore, tw, sign); break;
-        default: launch_sym<T, 512>(grid, s, buf, lstride, estride, B, par, nstore, tw, sign); break;
+void fft2d(C<T> *buf, int n0, int n1, int howmany, int sign, const C<T> *tw0, const C<T> *tw1, const FftPlan &p0,
+           const FftPlan &p1, cudaStream_t s, long *launches) {
+    fft_lines<T>(buf, n0, (long)n1 * howmany, howmany, howmany, n1, n1, p1, tw1, sign, s, launches);
+    fft_lines<T>(buf, n1, howmany, (long)n1 * howmany, howmany, n0, n0, p0, tw0, sign, s, launches);
+}
+
+template <int N>
+static void launch_sym(dim3 grid, cudaStream_t s, float2 *buf, long lstride, long estride, int B, float par, int nstore,
+                       const float2 *tw, int sign) {
+    reg_attr<float, N>((const void *)k_lines_sym_r<float, N>);
+    k_lines_sym_r<float, N><<<grid, reg_threads<N, float>(), reg_smem<N, float>(), s>>>(buf, lstride, estride, B, par,
+                                                                                        nstore, tw, sign);
+}
+
+template <> bool fft_lines_sym_ok<float>(const FftPlan &p, int) { return reg_fft_ok(p.n); }
+template <> bool fft_lines_sym_ok<double>(const FftPlan &p, int nlines) { return p.gen.ns > 0 && nlines <= 65535; }
+
+template <>
+void fft_lines_sym<float>(float2 *buf, int nlines, long lstride, long estride, int B, int parity, int nstore,
+                          const FftPlan &p, const float2 *tw, int sign, cudaStream_t s, long *launches) {
+    EGX_CHECK(reg_fft_ok(p.n), EGX_ERR_INVALID, "mirrored FFT lines need a length in {64, 128, 256, 512}");
+    dim3 grid(nlines, (B + RegCols<float>::BT - 1) / RegCols<float>::BT);
+    const float par = (float)parity;
+    switch (p.n) {
+        case 64: launch_sym<64>(grid, s, buf, lstride, estride, B, par, nstore, tw, sign); break;
+        case 128: launch_sym<128>(grid, s, buf, lstride, estride, B, par, nstore, tw, sign); break;
+        case 256: launch_sym<256>(grid, s, buf, lstride, estride, B, par, nstore, tw, sign); break;
+        default: launch_sym<512>(grid, s, buf, lstride, estride, B, par, nstore, tw, sign); break;
     }
     EGX_CUDA(cudaGetLastError());
     if (launches) *launches += 1;
 }
 
-template void fft_lines_sym<double>(C<double> *, int, long, long, int, int, int, int, const C<double> *, int,
-                                    cudaStream_t, long *);
-template void fft_lines_sym<float>(C<float> *, int, long, long, int, int, int, int, const C<float> *, int,
-                                   cudaStream_t, long *);
+template <>
+void fft_lines_sym<double>(double2 *buf, int nlines, long lstride, long estride, int B, int parity, int nstore,
+                           const FftPlan &p, const double2 *tw, int sign, cudaStream_t s, long *launches) {
+    EGX_CHECK(gen_lines_sym(p, buf, nlines, lstride, estride, B, parity, nstore, tw, sign, s), EGX_ERR_INVALID,
+              "mirrored FFT lines need a length with a generic plan");
+    EGX_CUDA(cudaGetLastError());
+    if (launches) *launches += 1;
+}
 
 template void fft_lines<double>(C<double> *, int, long, long, int, int, int, const FftPlan &, const C<double> *, int,
                                 cudaStream_t, long *);

@@ -90,14 +90,29 @@ template <typename T>
 void fft_lines(C<T> *buf, int nlines, long lstride, long estride, int B, int nload, int nstore, const FftPlan &p,
                const C<T> *tw, int sign, cudaStream_t s, long *launches);
 
-// DFTs of length n of lines stored by their first half: element e is
-// v[e] for e < n/2, 0 at n/2 and parity * v[n - e] beyond (a real-space
-// Green component and its mirror image); outputs e < nstore are written back
-// in place. Lengths with a register plan only (fft_lines_sym_ok).
-bool fft_lines_sym_ok(int n);
+// DFTs of lines stored by their first half: element e is v[e] for e < n/2, 0
+// at n/2 and parity * v[n - e] beyond (a real-space Green component and its
+// mirror image); outputs e < nstore are written back in place. Lengths that
+// fft_lines_sym_ok<T> takes: complex64 those with a register plan, complex128
+// those with a generic one.
+template <typename T> bool fft_lines_sym_ok(const FftPlan &p, int nlines);
 template <typename T>
-void fft_lines_sym(C<T> *buf, int nlines, long lstride, long estride, int B, int parity, int nstore, int n,
+void fft_lines_sym(C<T> *buf, int nlines, long lstride, long estride, int B, int parity, int nstore, const FftPlan &p,
                    const C<T> *tw, int sign, cudaStream_t s, long *launches);
+
+// The generic transform's passes (egx_fft_gen.cu); false, and nothing
+// launched, where the length has no such plan.
+template <typename T>
+bool gen_fwd_y(const FftPlan &p, const C<T> *x, const OperatorData<T> &op, C<T> *buf, const OpDims &d, const C<T> *tw,
+               cudaStream_t s);
+template <typename T>
+bool gen_bwd_y(const FftPlan &p, const C<T> *buf, const C<T> *x, const OperatorData<T> &op, C<T> *y, const OpDims &d,
+               const C<T> *tw, cudaStream_t s);
+template <typename T>
+bool gen_lines(const FftPlan &p, C<T> *buf, int nlines, long lstride, long estride, int B, int nload, int nstore,
+               const C<T> *tw, int sign, cudaStream_t s);
+bool gen_lines_sym(const FftPlan &p, double2 *buf, int nlines, long lstride, long estride, int B, int parity,
+                   int nstore, const double2 *tw, int sign, cudaStream_t s);
 
 // In-place batched 2-D DFT (egx_fft2d).
 template <typename T>

@@ -82,10 +82,10 @@ void gather_quadrant(int nx, int ny, int nz, const double *const comps[6], std::
         }
 }
 
-// The digit copy of a tensor, where the complex128 contraction takes it: with
-// a complex128 tensor, and on the first complex128 apply of a mixed one (its
-// inner solves do not read it). Without the memory for it the contraction
-// stays on the FP64 (or double-FP32) kernel.
+// The digit copy of a tensor, where the digit contraction takes it: with the
+// tensor, but for mixed ones in the sub-block layout on their first complex128
+// apply (their inner applies do not read it). Without the memory for it the
+// contraction stays on the kernels that need none.
 void make_digits(egx_ctx *ctx, egx_green *g) {
     if (g->dig.p || g->no_dig || !contract_dig_fits(g->nz)) return;
     GreenDims gd{g->nx, g->ny, g->nz};
@@ -375,7 +375,7 @@ void apply_dev(egx_ctx *ctx, const C<T> *x, C<T> *y, int nrhs, bool ds) {
     }
     op.type = ctx->type;
     if (dbl) make_digits(ctx, ctx->g);
-    op.dig = dbl ? ctx->g->dig.p : nullptr;
+    op.dig = ctx->g->dig.p;
     const C<T> *G = dbl ? (const C<T> *)ctx->g->g64.p : (const C<T> *)ctx->g->g32.p;
     const C<T> *tw0 = dbl ? (const C<T> *)ctx->tw0_64.p : (const C<T> *)ctx->tw0_32.p;
     const C<T> *tw1 = dbl ? (const C<T> *)ctx->tw1_64.p : (const C<T> *)ctx->tw1_32.p;
@@ -744,7 +744,7 @@ int egx_green_build(egx_ctx *ctx, const egx_model *model, double omega, int n_ha
         // the mixed form transforms the FP64 face integrals laterally in complex64
         build_green(gm, n_hankels, ctx->stream, g->g64, &st, &ctx->launches, &ctx->timers, &ctx->gws,
                     precision == EGX_PREC_MIXED);
-        if (precision != EGX_PREC_MIXED) make_digits(ctx, g.get());
+        if (precision != EGX_PREC_MIXED || !sb_layout(g->nz)) make_digits(ctx, g.get());
         if (precision == EGX_PREC_MIXED) {
             GreenDims gd{gm.nx, gm.ny, gm.nz};
             g->g32.swap(ctx->spare32);
@@ -773,7 +773,7 @@ int egx_green_upload(egx_ctx *ctx, int nx, int ny, int nz, const double *const c
         g->nz = nz;
         g->g64.ensure(q.size() * sizeof(cd));
         EGX_CUDA(cudaMemcpyAsync(g->g64.p, q.data(), q.size() * sizeof(cd), cudaMemcpyHostToDevice, ctx->stream));
-        if (precision != EGX_PREC_MIXED) make_digits(ctx, g.get());
+        if (precision != EGX_PREC_MIXED || !sb_layout(nz)) make_digits(ctx, g.get());
         if (precision == EGX_PREC_MIXED) {
             GreenDims gd{nx, ny, nz};
             g->g32.ensure(green_c64_entries(gd) * sizeof(float2));

@@ -44,7 +44,7 @@ struct OperatorData {
     const C<T> *fwd;  // [nz]
     const C<T> *bwd;  // [nz]
     int type;         // EGX_OP_A / EGX_OP_CHI0
-    const void *dig = nullptr;  // digit copy of the complex128 tensor (digitise)
+    const void *dig = nullptr;  // digit copy of the tensor (digitise)
 };
 
 // Launch the full apply y = K x (nrhs vectors) on `stream`.
@@ -57,13 +57,15 @@ void operator_apply(const OpDims &d, const OperatorData<T> &op, const C<T> *G, c
 // vectors fit in 96 KiB
 bool contract_ds_fits(int nz, int nrhs);
 
-// complex128 contraction with error-free digit products on the tensor cores
-// (egx_contract_dig.cu). It reads a copy of the tensor in digits that
-// digitise() makes once per tensor (contract_dig_bytes() of it).
+// contraction with error-free digit products on the tensor cores
+// (egx_contract_dig.cu): complex128, and complex64 of the packed layout. It
+// reads a copy of the tensor in digits that digitise() makes once per tensor
+// (contract_dig_bytes() of it).
 bool contract_dig_fits(int nz);
 size_t contract_dig_bytes(const GreenDims &gd);
 void digitise(const double2 *g64, void *out, const GreenDims &gd, cudaStream_t s, long *launches);
-void launch_contract_dig(double2 *buf, const void *dig, const OpDims &d, int *err, cudaStream_t s);
+template <typename T>
+void launch_contract_dig(C<T> *buf, const void *dig, const OpDims &d, int *err, cudaStream_t s);
 
 // complex64 contraction with TMA-staged blocks (egx_contract.cu); `err`
 // receives EGX_ERR_TIMEOUT if a bounded wait expires.

@@ -84,3 +84,36 @@ def test_zero_and_nonfinite_vectors(egx_ctx):
             assert np.array_equal(y[0], want) and not np.isfinite(y[1]).any()
     finally:
         g.free()
+
+
+# complex64: inputs and results round at 2^-24, the two transforms of 12 and 10
+# points at 2^-24 per stage (16 stages in all); the products are exact to
+# 2^-29 of the block's largest: (2 + 16) 2^-24 = 1.1e-6, doubled for the
+# stages' own constants.
+TOL_C64 = 2.2e-6
+
+
+@pytest.mark.parametrize("nz,nrhs", [(1, 2), (2, 1), (5, 3), (8, 2), (17, 1), (22, 2), (33, 1), (35, 4), (37, 2),
+                                     (39, 1), (47, 2), (49, 1)])
+@pytest.mark.parametrize("decades", [0, 6])
+def test_complex64_apply_by_digits_matches_oracle(egx_ctx, nz, nrhs, decades):
+    """Packed layouts, one and two right-hand sides per pass with a remainder."""
+    m = _model(nz, nz)
+    f = m.frequencies[1]
+    om = OmegaModel.build(m, f)
+    g = egx_ctx.green_build(m, freq_to_omega(f), 10)
+    G = g.download()
+    g.free()
+    rng = np.random.default_rng(nz)
+    G = _layer_scaled(G, nz, 10.0 ** rng.uniform(-decades / 2, decades / 2, nz))
+    g = egx_ctx.green_upload(G, m.nx, m.ny, nz, precision=egx.PREC_MIXED)
+    try:
+        egx_ctx.op_prepare(g, om.zeta, om.zeta0, m.layer_thickness, op.OP_A)
+        n = m.nx * m.ny * 3 * nz
+        xs = rng.standard_normal((nrhs, n)) + 1j * rng.standard_normal((nrhs, n))
+        xs = (xs * 10.0 ** rng.uniform(-3, 3, (nrhs, 1))).astype(np.complex64)
+        y = egx_ctx.op_apply_c64(xs.reshape(-1), nrhs=nrhs).reshape(nrhs, n)
+        for i in range(nrhs):
+            assert rel(y[i], op.apply(G, om, xs[i].astype(complex), op.OP_A)) < TOL_C64, i
+    finally:
+        g.free()

@@ -3,7 +3,7 @@
 // RightPreconditionerRequest plug point, Extreme.Fgmres/FlexibleGmresSolver.cs:24-36),
 // trained on (residual v, GMRES-preconditioner output) pairs that the solver
 // generates, with the forward and backward passes on BF16 tensor-core GEMMs
-// (mma.sync m16n8k16, FP32 accumulation) and Adam, all in this file.
+// (mma.sync m16n8k16 and tcgen05, FP32 accumulation) and Adam.
 //
 // Network, per sample on the nx x ny x nz anomaly mesh (depth is a spatial
 // axis), channels last; on the device sample b is stored as nz slices, row
@@ -23,8 +23,11 @@
 // Loss per batch: mean over samples of |Out - T|^2 / |T|^2 with T = (z* - v)
 // / rms(v) the target correction.
 //
-// Weights and activations are FP32 in memory; every GEMM converts its
-// operands to BF16 on the way into shared memory and accumulates in FP32.
+// Weights and activations are FP32 in memory; every product converts its
+// operands to BF16 on the way in and accumulates in FP32. The passes over
+// whole activations are in egx_learn_layer.cu (widths that are a multiple of
+// 4) and egx_learn_tc.cu (lift and projection); the strided GEMM here does
+// the products on retained modes, and every product of the other widths.
 #include <cuda_bf16.h>
 
 #include <cmath>
@@ -38,17 +41,15 @@ namespace egx {
 
 namespace {
 
-constexpr int KM = 16;  // retained modes per lateral direction
+constexpr int KM = kNetModes;
 
 // ------------------------------------------------------------------ GEMM
 // C[m, n] = alpha sum_k A[m, k] B[k, n] + beta C[m, n], batched over z with
 // arbitrary strides (transposes are strides): element (m, k) of batch b at
-// A[b a_b + m a_m + k a_k], likewise B (k, n) and C (m, n). With ksplit > 1
-// (batch 1) the z index splits K instead and the partial products are added
-// to C atomically (C zeroed by the caller): the weight gradients, whose K is
-// every row of the batch.
+// A[b a_b + m a_m + k a_k], likewise B (k, n) and C (m, n). The small products
+// of the network, and those of widths without 16-byte rows.
 struct GemmArgs {
-    int M, N, K, batch, ksplit;
+    int M, N, K, batch;
     const float *A;
     long a_m, a_k, a_b;
     const float *B;
@@ -71,13 +72,7 @@ __device__ __forceinline__ void mma_bf16(float *c, const uint32_t *a, uint32_t b
 __global__ void __launch_bounds__(128) k_gemm_bf16(const GemmArgs g) {
     __shared__ __align__(16) __nv_bfloat16 As[GBM][GBK + GPAD];  // (m, k)
     __shared__ __align__(16) __nv_bfloat16 Bs[GBN][GBK + GPAD];  // (n, k)
-    const int b = g.ksplit > 1 ? 0 : blockIdx.z;
-    int kbeg = 0, kend = g.K;
-    if (g.ksplit > 1) {
-        const int kc = ((g.K + g.ksplit - 1) / g.ksplit + GBK - 1) / GBK * GBK;
-        kbeg = blockIdx.z * kc;
-        kend = min(g.K, kbeg + kc);
-    }
+    const int b = blockIdx.z;
     const float *A = g.A + (long)b * g.a_b;
     const float *B = g.B + (long)b * g.b_b;
     float *C = g.C + (long)b * g.c_b;
@@ -97,16 +92,16 @@ __global__ void __launch_bounds__(128) k_gemm_bf16(const GemmArgs g) {
             for (int c = 0; c < 4; c++) acc[i][j][c] = 0.f;
     // loads run along whichever index is contiguous in memory
     const bool a_kfast = g.a_k == 1 || g.a_m != 1, b_kfast = g.b_k == 1 && g.b_n != 1;
-    for (int k0 = kbeg; k0 < kend; k0 += GBK) {
+    for (int k0 = 0; k0 < g.K; k0 += GBK) {
         for (int e = tid; e < GBM * GBK; e += 128) {
             const int m = a_kfast ? e / GBK : e % GBM, k = a_kfast ? e % GBK : e / GBM;
             const int gm = m0 + m, gk = k0 + k;
-            As[m][k] = __float2bfloat16_rn((gm < g.M && gk < kend) ? A[gm * g.a_m + gk * g.a_k] : 0.f);
+            As[m][k] = __float2bfloat16_rn((gm < g.M && gk < g.K) ? A[gm * g.a_m + gk * g.a_k] : 0.f);
         }
         for (int e = tid; e < GBN * GBK; e += 128) {
             const int n = b_kfast ? e / GBK : e % GBN, k = b_kfast ? e % GBK : e / GBN;
             const int gn = n0 + n, gk = k0 + k;
-            Bs[n][k] = __float2bfloat16_rn((gn < g.N && gk < kend) ? B[gk * g.b_k + gn * g.b_n] : 0.f);
+            Bs[n][k] = __float2bfloat16_rn((gn < g.N && gk < g.K) ? B[gk * g.b_k + gn * g.b_n] : 0.f);
         }
         __syncthreads();
 #pragma unroll
@@ -143,57 +138,35 @@ __global__ void __launch_bounds__(128) k_gemm_bf16(const GemmArgs g) {
                 if (m < g.M && n < g.N) {
                     float *p = C + m * g.c_m + n * g.c_n;
                     const float v = g.alpha * acc[i][j][c];
-                    if (g.ksplit > 1)
-                        atomicAdd(p, v);
-                    else
-                        *p = g.beta != 0.f ? v + g.beta * *p : v;
+                    *p = g.beta != 0.f ? v + g.beta * *p : v;
                 }
             }
 }
 
 void gemm(const GemmArgs &g, cudaStream_t s, long *launches) {
     const long tiles = (long)((g.M + GBM - 1) / GBM) * ((g.N + GBN - 1) / GBN);
-    EGX_CHECK(g.M >= 1 && g.N >= 1 && tiles <= 0x7fffffffL && g.batch <= 65535 && (g.ksplit <= 1 || g.batch == 1),
+    EGX_CHECK(g.M >= 1 && g.N >= 1 && tiles <= 0x7fffffffL && g.batch <= 65535,
               EGX_ERR_INVALID, "bad GEMM shape");
-    dim3 grid((unsigned)tiles, 1, g.ksplit > 1 ? g.ksplit : g.batch);
+    dim3 grid((unsigned)tiles, 1, g.batch);
     k_gemm_bf16<<<grid, 128, 0, s>>>(g);
     EGX_CUDA(cudaGetLastError());
     if (launches) ++*launches;
 }
 
 // -------------------------------------------------------------- elementwise
-__device__ __forceinline__ float gelu(float x) {
-    const float c = 0.7978845608028654f;  // sqrt(2/pi)
-    return 0.5f * x * (1.f + tanhf(c * (x + 0.044715f * x * x * x)));
-}
-__device__ __forceinline__ float gelu_d(float x) {
-    const float c = 0.7978845608028654f;
-    const float u = c * (x + 0.044715f * x * x * x), th = tanhf(u);
-    return 0.5f * (1.f + th) + 0.5f * x * (1.f - th * th) * c * (1.f + 3.f * 0.044715f * x * x);
-}
-
 // pre[r][c] += bias[c]; out = act ? gelu(pre) : pre
 __global__ void k_bias_act(float *pre, const float *__restrict__ bias, long rows, int cols, int act, float *out) {
     const long n = rows * cols;
     for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
         const float v = pre[i] + bias[i % cols];
         pre[i] = v;
-        out[i] = act ? gelu(v) : v;
+        out[i] = act ? net_gelu(v) : v;
     }
 }
 
 __global__ void k_gelu_bwd(float *d, const float *__restrict__ pre, long n) {
     for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x)
-        d[i] *= gelu_d(pre[i]);
-}
-
-// out[c] = sum_r x[r][c] (out zeroed by the caller)
-__global__ void k_colsum(const float *__restrict__ x, long rows, int cols, float *out) {
-    const int c = blockIdx.y * blockDim.x + threadIdx.x;
-    if (c >= cols) return;
-    float acc = 0.f;
-    for (long r = blockIdx.x; r < rows; r += gridDim.x) acc += x[r * cols + c];
-    atomicAdd(out + c, acc);
+        d[i] *= net_gelu_d(pre[i]);
 }
 
 // per-sample sum of |v|^2 over n complex entries (out zeroed by the caller)
@@ -288,14 +261,27 @@ __global__ void k_loss_sums(const float *__restrict__ out, const float *__restri
     }
 }
 
-// dOut = 2 (Out - T) / (batch |T_b|^2)
+// dOut = 2 (Out - T) / (batch |T_b|^2). The difference and the factor are
+// unevaluated sums of two floats, so that the result alone is rounded; the
+// FP64 form (two operations per clock and SM, a division per entry) is left
+// for results outside the normal range. 25 M entries (8 samples of
+// 128x128x32): 110 us, FP64 alone 696.
 __global__ void k_loss_grad(const float *__restrict__ out, const float *__restrict__ T, const double *t2,
                             long per_sample, int batch, float *dout) {
-    const long total = per_sample * batch;
-    for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long)gridDim.x * blockDim.x) {
-        const int b = (int)(i / per_sample);
-        const double den = t2[b] > 0 ? (double)batch * t2[b] : 1.0;
-        dout[i] = (float)(2.0 * ((double)out[i] - T[i]) / den);
+    const int b = blockIdx.y;
+    const double den = t2[b] > 0 ? (double)batch * t2[b] : 1.0;
+    // 2 / den = (fh + fl) 2^e with fh in [1, 2)
+    const double f = 2.0 / den;
+    const int e = f > 0 ? max(-1000, min(1000, ilogb(f))) : 0;
+    const double m = scalbn(f, -e);
+    const float fh = (float)m, fl = (float)(m - fh);
+    for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < per_sample; i += (long)gridDim.x * blockDim.x) {
+        const float x = out[b * per_sample + i], y = T[b * per_sample + i];
+        const float d = x - y, u = d - x, dl = (x - (d - u)) - (y + u);
+        const float p = d * fh, pe = __fmaf_rn(d, fh, -p);
+        float r = ldexpf(p + (pe + __fmaf_rn(d, fl, dl * fh)), e);
+        if (!(fabsf(r) >= 1.1754944e-38f && fabsf(r) <= 3.4028235e38f)) r = (float)(2.0 * ((double)x - y) / den);
+        dout[b * per_sample + i] = r;
     }
 }
 
@@ -322,6 +308,7 @@ struct egx_net {
     int nx = 0, ny = 0, nz = 0, W = 0, L = 0, cin = 0, cout = 0;
     long ncell = 0, n_params = 0;
     int nmodels = 0;  // conductivity models set (sample b uses model b % nmodels)
+    bool fused = false;  // the layers' passes by egx_learn_layer.cu
     int tc = 1;       // pointwise GEMMs on the tcgen05 kernel (egx_net_use_tcgen05)
     int *err = nullptr;  // the context's device error flag
     long off_P = 0, off_bP = 0, off_Q = 0, off_bQ = 0;
@@ -349,7 +336,7 @@ void ensure_batch(egx_net *n, int batch) {
     n->dOut.ensure(rows * n->cout * sizeof(float));
     for (int l = 0; l <= n->L; l++) n->H[l].ensure(rows * W * sizeof(float));
     for (int l = 0; l < n->L; l++) {
-        n->Pre[l].ensure(rows * W * sizeof(float));
+        if (!n->fused || l < n->L - 1) n->Pre[l].ensure(rows * W * sizeof(float));
         n->U[l].ensure((size_t)S * KM * KM * W * sizeof(float));
     }
     n->U1.ensure((size_t)S * KM * n->ny * W * sizeof(float));
@@ -373,13 +360,7 @@ GemmArgs ga(int M, int N, int K, int batch, const float *A, long a_m, long a_k, 
     g.A = A, g.a_m = a_m, g.a_k = a_k, g.a_b = a_b;
     g.B = B, g.b_k = b_k, g.b_n = b_n, g.b_b = b_b;
     g.C = C, g.c_m = c_m, g.c_n = c_n, g.c_b = c_b;
-    g.alpha = 1.f, g.beta = beta, g.ksplit = 1;
-    return g;
-}
-
-// a weight gradient: K = all rows, split over CTAs, added atomically
-GemmArgs wgrad(GemmArgs g) {
-    g.ksplit = (int)std::min<long>(256, std::max<long>(1, (long)g.K / 512));
+    g.alpha = 1.f, g.beta = beta;
     return g;
 }
 
@@ -387,35 +368,46 @@ GemmArgs wgrad(GemmArgs g) {
 // the tcgen05 kernel (egx_learn_tc.cu), or on the warp-level kernel when the
 // network's tcgen05 path is off or the width exceeds 32
 void pw(egx_net *n, int M, int K, const float *A, const float *B, long b_k, long b_n, int N, float *C, bool acc,
-        cudaStream_t s, long *launches) {
+        const float *bias, cudaStream_t s, long *launches) {
     if (n->tc && pw_gemm_tc_fits(K, N)) {
-        pw_gemm_tc(A, M, K, B, b_k, b_n, N, C, acc, n->err, s);
+        pw_gemm_tc(A, M, K, B, b_k, b_n, N, C, acc, bias, n->err, s);
         if (launches) ++*launches;
     } else {
         gemm(ga(M, N, K, 1, A, K, 1, 0, B, b_k, b_n, 0, C, N, 1, 0, acc ? 1.f : 0.f), s, launches);
+        if (bias) {
+            k_bias_act<<<blocks_for((long)M * N), 256, 0, s>>>(C, bias, M, N, 0, C);
+            if (launches) ++*launches;
+        }
     }
 }
 
-// X0 (encoded) -> Out; keeps the activations for backward. The B samples
-// are B nz depth slices for the lateral operations.
-void forward(egx_net *n, int B, cudaStream_t s, long *launches) {
+// X0 (encoded) -> Out; keeps the activations for backward (keep: the layers'
+// sums before the activation too). The B samples are B nz depth slices for
+// the lateral operations.
+void forward(egx_net *n, int B, bool keep, cudaStream_t s, long *launches) {
     const int nx = n->nx, ny = n->ny, W = n->W, nz = n->nz;
     const int S = B * nz;
     const long rows = (long)S * n->ncell, slab = n->ncell * W;
     const float *bx = n->bx.as<float>(), *by = n->by.as<float>();
-    pw(n, (int)rows, n->cin, n->X0.as<float>(), n->p(n->off_P), W, 1, W, n->H[0].as<float>(), false, s, launches);
-    k_bias_act<<<blocks_for(rows * W), 256, 0, s>>>(n->H[0].as<float>(), n->p(n->off_bP), rows, W, 0,
-                                                     n->H[0].as<float>());
+    // the batched products' grids
+    EGX_CHECK((long)S * std::max(nx, KM) <= 65535, EGX_ERR_INVALID, "bad GEMM shape");
+    pw(n, (int)rows, n->cin, n->X0.as<float>(), n->p(n->off_P), W, 1, W, n->H[0].as<float>(), false, n->p(n->off_bP), s,
+       launches);
     for (int l = 0; l < n->L; l++) {
         const float *Hl = n->H[l].as<float>();
         float *U1 = n->U1.as<float>(), *Ul = n->U[l].as<float>(), *V = n->V.as<float>(), *S1 = n->S1.as<float>();
         float *Pre = n->Pre[l].as<float>();
+        const bool act = l < n->L - 1;
         // U1[s] = Bx^T H[s]                     (KM x ny W) per depth slice s
-        gemm(ga(KM, ny * W, nx, S, bx, 1, KM, 0, Hl, (long)ny * W, 1, (long)nx * ny * W, U1, (long)ny * W, 1,
-                (long)KM * ny * W),
-             s, launches);
         // U[s, i] = By^T U1[s, i]              (KM x W)
-        gemm(ga(KM, W, ny, S * KM, by, 1, KM, 0, U1, W, 1, (long)ny * W, Ul, W, 1, (long)KM * W), s, launches);
+        if (n->fused) {
+            net_analysis(bx, nx, Hl, (long)ny * W, slab, S, ny * W, U1, s, launches);
+            net_analysis(by, ny, U1, W, (long)ny * W, (long)S * KM, W, Ul, s, launches);
+        } else {
+            gemm(ga(KM, ny * W, nx, S, bx, 1, KM, 0, Hl, (long)ny * W, 1, slab, U1, (long)ny * W, 1, (long)KM * ny * W),
+                 s, launches);
+            gemm(ga(KM, W, ny, S * KM, by, 1, KM, 0, U1, W, 1, (long)ny * W, Ul, W, 1, (long)KM * W), s, launches);
+        }
         // V[:, mode] = U[:, mode] Wm[mode]      (S x W) per mode
         gemm(ga(S, W, W, KM * KM, Ul, (long)KM * KM * W, 1, W, n->p(n->off_Wm[l]), W, 1, (long)W * W, V,
                 (long)KM * KM * W, 1, W),
@@ -424,30 +416,31 @@ void forward(egx_net *n, int B, cudaStream_t s, long *launches) {
         gemm(ga(nx, KM * W, KM, S, bx, KM, 1, 0, V, (long)KM * W, 1, (long)KM * KM * W, S1, (long)KM * W, 1,
                 (long)nx * KM * W),
              s, launches);
-        // Pre[s, x] = By S1[s, x]               (ny x W)
+        // Pre[s, x] = By S1[s, x] + H Wp + Dz H + b, and its activation
+        if (n->fused) {
+            NetLayer a;
+            a.in = Hl, a.sp = S1, a.bas = by, a.D = n->p(n->off_Dz[l]), a.Wt = n->p(n->off_Wp[l]);
+            a.bias = n->p(n->off_b[l]), a.pre = keep && act ? Pre : nullptr, a.out = n->H[l + 1].as<float>();
+            a.d_o = nz, a.d_i = 1, a.w_k = W, a.w_n = 1;
+            a.sp_s = (long)nx * KM * W, a.sp_o = (long)KM * W, a.sp_j = W;
+            a.ncell = n->ncell, a.o_stride = ny, a.l_stride = 1;
+            a.batch = B, a.nz = nz, a.W = W, a.n_outer = nx, a.n_line = ny, a.act = act;
+            net_layer(a, s, launches);
+            continue;
+        }
         gemm(ga(ny, W, KM, S * nx, by, KM, 1, 0, S1, W, 1, (long)KM * W, Pre, W, 1, (long)ny * W), s, launches);
-        // Pre += H Wp
-        pw(n, (int)rows, W, Hl, n->p(n->off_Wp[l]), W, 1, W, Pre, true, s, launches);
+        pw(n, (int)rows, W, Hl, n->p(n->off_Wp[l]), W, 1, W, Pre, true, nullptr, s, launches);
         // Pre[b, z] += sum_z' Dz[z, z'] H[b, z']   (nz x ncell W) per sample
         gemm(ga(nz, (int)slab, nz, B, n->p(n->off_Dz[l]), nz, 1, 0, Hl, slab, 1, (long)nz * slab, Pre, slab, 1,
                 (long)nz * slab, 1.f),
              s, launches);
-        k_bias_act<<<blocks_for(rows * W), 256, 0, s>>>(Pre, n->p(n->off_b[l]), rows, W, l < n->L - 1 ? 1 : 0,
+        k_bias_act<<<blocks_for(rows * W), 256, 0, s>>>(Pre, n->p(n->off_b[l]), rows, W, act ? 1 : 0,
                                                          n->H[l + 1].as<float>());
         if (launches) ++*launches;
     }
-    pw(n, (int)rows, W, n->H[n->L].as<float>(), n->p(n->off_Q), n->cout, 1, n->cout, n->Out.as<float>(), false, s,
-       launches);
-    k_bias_act<<<blocks_for(rows * n->cout), 256, 0, s>>>(n->Out.as<float>(), n->p(n->off_bQ), rows, n->cout, 0,
-                                                           n->Out.as<float>());
-    if (launches) *launches += 2;
+    pw(n, (int)rows, W, n->H[n->L].as<float>(), n->p(n->off_Q), n->cout, 1, n->cout, n->Out.as<float>(), false,
+       n->p(n->off_bQ), s, launches);
     EGX_CUDA(cudaGetLastError());
-}
-
-void colsum(const float *x, long rows, int cols, float *out, cudaStream_t s, long *launches) {
-    dim3 grid((unsigned)std::min<long>(rows, 1024), (cols + 127) / 128);
-    k_colsum<<<grid, 128, 0, s>>>(x, rows, cols, out);
-    if (launches) ++*launches;
 }
 
 // dOut -> grads (zeroed here)
@@ -459,28 +452,34 @@ void backward(egx_net *n, int B, cudaStream_t s, long *launches) {
     EGX_CUDA(cudaMemsetAsync(n->grads.p, 0, n->n_params * sizeof(float), s));
     float *dOut = n->dOut.as<float>();
     // dQ = H_L^T dOut, dbQ, dH = dOut Q^T
-    gemm(wgrad(ga(W, n->cout, (int)rows, 1, n->H[n->L].as<float>(), 1, W, 0, dOut, n->cout, 1, 0, n->gr(n->off_Q),
-                  n->cout, 1, 0)),
-         s, launches);
-    colsum(dOut, rows, n->cout, n->gr(n->off_bQ), s, launches);
-    pw(n, (int)rows, n->cout, dOut, n->p(n->off_Q), 1, n->cout, W, n->dH.as<float>(), false, s, launches);
+    net_weight_grad(n->H[n->L].as<float>(), W, dOut, n->cout, rows, nullptr, n->gr(n->off_Q), n->gr(n->off_bQ), s,
+                    launches);
+    pw(n, (int)rows, n->cout, dOut, n->p(n->off_Q), 1, n->cout, W, n->dH.as<float>(), false, nullptr, s, launches);
     for (int l = n->L - 1; l >= 0; l--) {
         float *dPre = n->dH.as<float>(), *dH2 = n->dH2.as<float>();
         const float *Hl = n->H[l].as<float>(), *Ul = n->U[l].as<float>();
-        if (l < n->L - 1) {
-            k_gelu_bwd<<<blocks_for(rows * W), 256, 0, s>>>(dPre, n->Pre[l].as<float>(), rows * W);
+        const float *pre = l < n->L - 1 ? n->Pre[l].as<float>() : nullptr;
+        // dPre = dH act'(Pre), db, dWp = H^T dPre: one pass where one column of
+        // tiles covers the width
+        if (pre && !(n->fused && W <= 32)) {
+            k_gelu_bwd<<<blocks_for(rows * W), 256, 0, s>>>(dPre, pre, rows * W);
             if (launches) ++*launches;
+            pre = nullptr;
         }
-        colsum(dPre, rows, W, n->gr(n->off_b[l]), s, launches);
-        // dWp = H^T dPre; dH2 = dPre Wp^T
-        gemm(wgrad(ga(W, W, (int)rows, 1, Hl, 1, W, 0, dPre, W, 1, 0, n->gr(n->off_Wp[l]), W, 1, 0)), s, launches);
-        pw(n, (int)rows, W, dPre, n->p(n->off_Wp[l]), 1, W, W, dH2, false, s, launches);
+        net_weight_grad(Hl, W, dPre, W, rows, pre, n->gr(n->off_Wp[l]), n->gr(n->off_b[l]), s, launches);
+        // dDz[z, z'] = sum over samples and (cell, channel) of dPre[b, z] H[b, z']
+        net_depth_grad(dPre, Hl, nz, slab, B, n->gr(n->off_Dz[l]), s, launches);
         // spectral branch
         float *dS1 = n->dS1.as<float>(), *dV = n->dV.as<float>(), *dU = n->dU.as<float>(), *dU1 = n->dU1.as<float>();
-        gemm(ga(KM, W, ny, S * nx, by, 1, KM, 0, dPre, W, 1, (long)ny * W, dS1, W, 1, (long)KM * W), s, launches);
-        gemm(ga(KM, KM * W, nx, S, bx, 1, KM, 0, dS1, (long)KM * W, 1, (long)nx * KM * W, dV, (long)KM * W, 1,
-                (long)KM * KM * W),
-             s, launches);
+        if (n->fused) {
+            net_analysis(by, ny, dPre, W, (long)ny * W, (long)S * nx, W, dS1, s, launches);
+            net_analysis(bx, nx, dS1, (long)KM * W, (long)nx * KM * W, S, KM * W, dV, s, launches);
+        } else {
+            gemm(ga(KM, W, ny, S * nx, by, 1, KM, 0, dPre, W, 1, (long)ny * W, dS1, W, 1, (long)KM * W), s, launches);
+            gemm(ga(KM, KM * W, nx, S, bx, 1, KM, 0, dS1, (long)KM * W, 1, (long)nx * KM * W, dV, (long)KM * W, 1,
+                    (long)KM * KM * W),
+                 s, launches);
+        }
         gemm(ga(W, W, S, KM * KM, Ul, 1, (long)KM * KM * W, W, dV, (long)KM * KM * W, 1, W, n->gr(n->off_Wm[l]), W,
                 1, (long)W * W),
              s, launches);
@@ -488,26 +487,30 @@ void backward(egx_net *n, int B, cudaStream_t s, long *launches) {
                 (long)KM * KM * W, 1, W),
              s, launches);
         gemm(ga(ny, W, KM, S * KM, by, KM, 1, 0, dU, W, 1, (long)KM * W, dU1, W, 1, (long)ny * W), s, launches);
-        gemm(ga(nx, ny * W, KM, S, bx, KM, 1, 0, dU1, (long)ny * W, 1, (long)KM * ny * W, dH2, (long)ny * W, 1,
-                (long)nx * ny * W, 1.f),
-             s, launches);
-        // depth mixing: dH2[b, z'] += sum_z Dz[z, z'] dPre[b, z]; dDz[z, z'] =
-        // sum over samples and (cell, channel) of dPre[b, z] H[b, z'] (each
-        // sample's product added into the gradient)
-        gemm(ga(nz, (int)slab, nz, B, n->p(n->off_Dz[l]), 1, nz, 0, dPre, slab, 1, (long)nz * slab, dH2, slab, 1,
-                (long)nz * slab, 1.f),
-             s, launches);
-        for (int b = 0; b < B; b++)
-            gemm(wgrad(ga(nz, nz, (int)slab, 1, dPre + (long)b * nz * slab, slab, 1, 0, Hl + (long)b * nz * slab, 1,
-                          slab, 0, n->gr(n->off_Dz[l]), nz, 1, 0, 1.f)),
+        // dH[b, z'] = Bx dU1 + dPre Wp^T + sum_z Dz[z, z'] dPre[b, z]
+        if (n->fused) {
+            NetLayer a;
+            a.in = dPre, a.sp = dU1, a.bas = bx, a.D = n->p(n->off_Dz[l]), a.Wt = n->p(n->off_Wp[l]);
+            a.bias = nullptr, a.pre = nullptr, a.out = dH2;
+            a.d_o = 1, a.d_i = nz, a.w_k = 1, a.w_n = W;
+            a.sp_s = (long)KM * ny * W, a.sp_o = W, a.sp_j = (long)ny * W;
+            a.ncell = n->ncell, a.o_stride = 1, a.l_stride = ny;
+            a.batch = B, a.nz = nz, a.W = W, a.n_outer = ny, a.n_line = nx, a.act = false;
+            net_layer(a, s, launches);
+        } else {
+            pw(n, (int)rows, W, dPre, n->p(n->off_Wp[l]), 1, W, W, dH2, false, nullptr, s, launches);
+            gemm(ga(nx, ny * W, KM, S, bx, KM, 1, 0, dU1, (long)ny * W, 1, (long)KM * ny * W, dH2, (long)ny * W, 1,
+                    (long)nx * ny * W, 1.f),
                  s, launches);
+            gemm(ga(nz, (int)slab, nz, B, n->p(n->off_Dz[l]), 1, nz, 0, dPre, slab, 1, (long)nz * slab, dH2, slab, 1,
+                    (long)nz * slab, 1.f),
+                 s, launches);
+        }
         n->dH.swap(n->dH2);
     }
     // dP = X0^T dH0, dbP
-    gemm(wgrad(ga(n->cin, W, (int)rows, 1, n->X0.as<float>(), 1, n->cin, 0, n->dH.as<float>(), W, 1, 0,
-                  n->gr(n->off_P), W, 1, 0)),
-         s, launches);
-    colsum(n->dH.as<float>(), rows, W, n->gr(n->off_bP), s, launches);
+    net_weight_grad(n->X0.as<float>(), n->cin, n->dH.as<float>(), W, rows, nullptr, n->gr(n->off_P), n->gr(n->off_bP),
+                    s, launches);
     EGX_CUDA(cudaGetLastError());
 }
 
@@ -533,7 +536,7 @@ void net_apply(egx_net *n, const float2 *v, float2 *z, int batch, cudaStream_t s
     EGX_CHECK(n->logsig.p, EGX_ERR_STATE, "learned preconditioner has no model (egx_net_set_model)");
     ensure_batch(n, batch);
     encode(n, v, batch, s, launches);
-    forward(n, batch, s, launches);
+    forward(n, batch, false, s, launches);
     const float *rms = n->scal.as<float>() + batch;
     k_decode<<<blocks_for((long)batch * n->ncell * 3 * n->nz), 256, 0, s>>>(v, rms, n->Out.as<float>(), n->ncell,
                                                                             n->nz, batch, z);
@@ -558,6 +561,7 @@ int egx_net_create(egx_ctx *ctx, int nx, int ny, int nz, int width, int layers, 
         auto n = std::unique_ptr<egx_net>(new egx_net());
         n->nx = nx, n->ny = ny, n->nz = nz, n->W = width, n->L = layers;
         n->err = ctx->errflag.as<int>();
+        n->fused = net_layer_fits(nz, width);
         n->cin = 7, n->cout = 6, n->ncell = (long)nx * ny;
         long off = 0;
         auto take = [&](long k) {
@@ -693,13 +697,13 @@ int egx_net_loss_grad(egx_ctx *ctx, egx_net *net, const float *v, const float *t
         const float *inv = net->scal.as<float>();
         k_encode_target<<<blocks_for((long)batch * net->nz * net->ncell * net->cout), 256, 0, s>>>(dt, inv, net->ncell, net->nz,
                                                                                          batch, net->T.as<float>());
-        forward(net, batch, s, &ctx->launches);
+        forward(net, batch, true, s, &ctx->launches);
         const long per = (long)net->nz * net->ncell * net->cout;  // one sample's outputs
         double *e2 = net->sums.as<double>() + batch, *t2 = e2 + batch;
         EGX_CUDA(cudaMemsetAsync(e2, 0, 2 * batch * sizeof(double), s));
         k_loss_sums<<<dim3((unsigned)std::min<long>((per + 255) / 256, 512), batch), 256, 0, s>>>(
             net->Out.as<float>(), net->T.as<float>(), per, e2, t2);
-        k_loss_grad<<<blocks_for(per * batch), 256, 0, s>>>(net->Out.as<float>(), net->T.as<float>(), t2, per, batch,
+        k_loss_grad<<<dim3((unsigned)std::min<long>((per + 255) / 256, 1024), batch), 256, 0, s>>>(net->Out.as<float>(), net->T.as<float>(), t2, per, batch,
                                                             net->dOut.as<float>());
         ctx->launches += 3;
         backward(net, batch, s, &ctx->launches);

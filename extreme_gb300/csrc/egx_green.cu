@@ -7,7 +7,9 @@
 // cell into sparse weight lists.
 // Device, per tensor half (asym: xz, yz; symm: xx, xy, yy, zz):
 //   k_layers   per lambda: eta, exp, P/Q reflection recursions of both modes
-//              (PlanCalculatorFast.cs:203-318, green_scalar.c:30-41);
+//              (PlanCalculatorFast.cs:203-318, green_scalar.c:30-41), once for
+//              both halves, with k_chain_factors and k_decays what of the
+//              kernels depends on one layer;
 //   k_kernels  per (transceiver, lambda): exponential sums, propagators and
 //              the kernels U1..U5 with their pre-Hankel normalisation
 //              (VolumeToVolumeCalculatorUFast.cs:34-337, green_scalar.c:86-386,
@@ -83,7 +85,10 @@ struct LayerArgs {
 };
 
 // Per lambda: eta, exp, P1, Q1, Ps, Qs over all layers. Arrays [6][L][nl]
-// (of the ten that k_chain_factors completes).
+// (of the thirteen that k_chain_factors completes). A serial chain of FP64
+// divisions over the layers per lambda and mode (grid y): bound by latency, so
+// all plan items' lambdas go in one launch, in small blocks (5,350 lambdas,
+// 7 layers: 102 us; 20 launches of five blocks took 3,010).
 __global__ void k_layers(const double *__restrict__ lam, int nl, const LayerArgs a, double2 *__restrict__ out) {
     int m = blockIdx.x * blockDim.x + threadIdx.x;
     if (m >= nl) return;
@@ -98,13 +103,14 @@ __global__ void k_layers(const double *__restrict__ lam, int nl, const LayerArgs
         eta[k] = dsqrt(dmk(l * l - v.x, -v.y));
         ex[k] = dexp(dscal(-2.0 * a.thick[k], eta[k]));
     }
-    double2 *Eta = out, *Ex = out + (long)L * nl, *P1 = out + 2L * L * nl, *Q1 = out + 3L * L * nl;
-    double2 *Ps = out + 4L * L * nl, *Qs = out + 5L * L * nl;
-    for (int k = 0; k < L; k++) {
-        Eta[(long)k * nl + m] = eta[k];
-        Ex[(long)k * nl + m] = ex[k];
-    }
-    for (int mode = 0; mode < 2; mode++) {
+    double2 *Eta = out, *Ex = out + (long)L * nl;
+    const int mode = blockIdx.y;
+    if (mode == 0)
+        for (int k = 0; k < L; k++) {
+            Eta[(long)k * nl + m] = eta[k];
+            Ex[(long)k * nl + m] = ex[k];
+        }
+    {
         double2 p[kMaxLayers], q[kMaxLayers];
         for (int k = 0; k < L; k++) p[k] = q[k] = dmk(0, 0);
         if (mode == 0) p[1] = ddiv(dsub(eta[1], eta[0]), dadd(eta[1], eta[0]));
@@ -132,7 +138,7 @@ __global__ void k_layers(const double *__restrict__ lam, int nl, const LayerArgs
             double2 part = dmul(be, ddiv(dsub(qexp, dmk(1, 0)), dadd(qexp, dmk(1, 0))));
             q[k - 1] = ddiv(dadd(dmk(1, 0), part), dsub(dmk(1, 0), part));
         }
-        double2 *P = mode == 0 ? P1 : Ps, *Q = mode == 0 ? Q1 : Qs;
+        double2 *P = out + (2L + 2 * mode) * L * nl, *Q = out + (3L + 2 * mode) * L * nl;
         for (int k = 0; k < L; k++) {
             P[(long)k * nl + m] = p[k];
             Q[(long)k * nl + m] = q[k];
@@ -143,41 +149,69 @@ __global__ void k_layers(const double *__restrict__ lam, int nl, const LayerArgs
 struct Trans {
     double r1, r2, s1, s2;
     int r, s;      // background layers of receiver / transmitter
+    int rc, tr;    // their anomaly layers
     int kase;      // 0 match, 1 receiver below, 2 receiver above
 };
 
 // The propagator chains' per-layer pieces, which depend on the layer and
 // lambda only (not on the transmitter pair): per mode (P1/Q1, Ps/Qs) the
-// head H[b] = 1 / (eta_b (1 - P_b Q_b X_b)) and the factors
-// F[k] = (1 + P_{k+1}) / (1 + P_k X_k) exp(z_{k+1} (eta_{k+1} - eta_k)),
-// so that a pair's chain A[t, b] = F[t] (... (F[b-1] H[b])) is a few complex
-// products. Arrays [mode][L][nl] after the six of k_layers: F at 6L nl, H at
-// 8L nl.
+// head H[b] = 1 / (eta_b (1 - P_b Q_b X_b)), the ratios G[k] =
+// (1 + P_{k+1}) / (1 + P_k X_k), and F[k] = G[k] exp(z_{k+1} (eta_{k+1} -
+// eta_k)), so that a pair's chain A[t, b] = F[t] (... (F[b-1] H[b])) is a few
+// complex products; and the decay across a layer, Y[k] = exp(-(z_{k+1} - z_k)
+// eta_k). Arrays [mode][L][nl] after the six of k_layers: F at 6L nl, H at
+// 8L nl, G at 10L nl, then Y [L][nl] at 12L nl. A thread per layer and lambda.
+constexpr int kLayArrays = 13;
 __global__ void k_chain_factors(int nl, const LayerArgs a, double2 *__restrict__ lay) {
     const int m = blockIdx.x * blockDim.x + threadIdx.x;
     if (m >= nl) return;
-    const int L = a.L;
-    const double2 *Eta = lay, *Ex = lay + (long)L * nl;
-    auto E = [&](int k) { return Eta[(long)k * nl + m]; };
+    const int L = a.L, k = blockIdx.y;
+    const long o = (long)k * nl + m;
+    const double2 ek = lay[o], xk = lay[(long)L * nl + o];
+    if (k + 1 < L) lay[12L * L * nl + o] = dexp(dscal(-(a.tops[k + 1] - a.tops[k]), ek));
+    double2 ez = dmk(0, 0);
+    if (k + 1 < L) ez = dexp(dscal(a.tops[k + 1], dsub(lay[o + nl], ek)));
     for (int mode = 0; mode < 2; mode++) {
         const double2 *P = lay + (2L + 2 * mode) * L * nl, *Q = lay + (3L + 2 * mode) * L * nl;
-        double2 *F = lay + (6L + mode) * L * nl, *H = lay + (8L + mode) * L * nl;
-        for (int b = 0; b < L; b++)
-            H[(long)b * nl + m] = drecip(dmul(E(b), dsub(dmk(1, 0), dmul(dmul(P[(long)b * nl + m], Q[(long)b * nl + m]),
-                                                                       Ex[(long)b * nl + m]))));
-        for (int k = 0; k + 1 < L; k++) {
-            const double2 num = dadd(dmk(1, 0), P[(long)(k + 1) * nl + m]);
-            const double2 den = dadd(dmk(1, 0), dmul(P[(long)k * nl + m], Ex[(long)k * nl + m]));
-            F[(long)k * nl + m] = dmul(ddiv(num, den), dexp(dscal(a.tops[k + 1], dsub(E(k + 1), E(k)))));
+        lay[(8L + mode) * L * nl + o] = drecip(dmul(ek, dsub(dmk(1, 0), dmul(dmul(P[o], Q[o]), xk))));
+        if (k + 1 < L) {
+            const double2 g = ddiv(dadd(dmk(1, 0), P[o + nl]), dadd(dmk(1, 0), dmul(P[o], xk)));
+            lay[(10L + mode) * L * nl + o] = g;
+            lay[(6L + mode) * L * nl + o] = dmul(g, ez);
         }
     }
 }
 
+// Per anomaly layer [z1, z2] (in background layer k, [z_k, z_{k+1}]) and
+// lambda, e = eta_k: f = 1 - exp(-(z2 - z1) e), u = exp(-(z1 - z_k) e), d =
+// exp(-(z_{k+1} - z2) e). Arrays [3][nz][nl]; the layer's own transmitter
+// entry in `trans` (rc = tr) is at diag[layer].
+__global__ void k_decays(int nl, const double2 *__restrict__ lay, const LayerArgs a, const Trans *__restrict__ trans,
+                         const int *__restrict__ diag, int nz, double2 *__restrict__ dec) {
+    const int m = blockIdx.x * blockDim.x + threadIdx.x;
+    if (m >= nl) return;
+    const int z = blockIdx.y;
+    const Trans T0 = trans[diag[z]];
+    const double2 e = lay[(long)T0.s * nl + m];
+    const long o = (long)z * nl + m, st = (long)nz * nl;
+    dec[o] = dsub(dmk(1, 0), dexp(dscal(-(T0.s2 - T0.s1), e)));
+    dec[st + o] = dexp(dscal(-(T0.s1 - a.tops[T0.s]), e));
+    dec[2 * st + o] = dexp(dscal(-(a.tops[T0.s + 1] - T0.s2), e));
+}
+
 // which kernels: bit0 U1, bit1 U2, bit2 U3, bit3 U4, bit4 U5; outputs packed
-// in that order, each [ntrans][nl_total] at column offset `col0`.
-__global__ void k_kernels(const double *__restrict__ lam, int nl, const double2 *__restrict__ lay, const LayerArgs a,
-                          const Trans *__restrict__ trans, int ntrans, int which, double2 *__restrict__ U,
-                          long nl_total, long col0) {
+// in that order, each [ntrans][nl].
+//
+// The exponential sums come from the decays of k_decays and k_chain_factors:
+// with the chain's exp(z_{k+1} (eta_{k+1} - eta_k)) multiplied out, every term
+// of a pair is a product of decays within the receiver's and transmitter's
+// layers and across the layers between, none of them above one. An
+// exponential is left for pairs in one background layer. FP64 pipes: 3.7 ms
+// for both tensor halves at 32 layers and 5,350 lambdas, against 8.0 with six
+// complex exponentials per pair and lambda.
+__global__ void k_kernels(const double *__restrict__ lam, int nl, const double2 *__restrict__ lay,
+                          const double2 *__restrict__ dec, int nz, const LayerArgs a, const Trans *__restrict__ trans,
+                          int ntrans, int which, double2 *__restrict__ U) {
     long idx = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= (long)ntrans * nl) return;
     const int tr = (int)(idx / nl);
@@ -188,72 +222,46 @@ __global__ void k_kernels(const double *__restrict__ lam, int nl, const double2 
     const double2 *Ps = lay + 4L * L * nl, *Qs = lay + 5L * L * nl;
 #define E(k) Eta[(long)(k) * nl + m]
     const int r = T0.r, s = T0.s, t = min(r, s), b = max(r, s);
-    const double dt = a.tops[t], db1 = a.tops[b + 1];
-    const double r1 = T0.r1, r2 = T0.r2, s1 = T0.s1, s2 = T0.s2;
-    const double2 er = E(r), es = E(s), et = E(t), eb = E(b);
+    const double r1 = T0.r1, r2 = T0.r2;
+    const double2 er = E(r), es = E(s);
     const double l = lam[m];
-    auto lin3 = [](double c1, double2 v1, double c2, double2 v2, double c3, double2 v3) {
-        double2 acc = dscal(c1, v1);
-        acc = dadd(acc, dscal(c2, v2));
-        return dadd(acc, dscal(c3, v3));
-    };
-    auto lin2 = [](double c1, double2 v1, double c2, double2 v2) { return dadd(dscal(c1, v1), dscal(c2, v2)); };
-    // CalculateT / CalculateR and the C, D sums. Each is a signed sum of four
-    // exponentials of the form e^G (e^a - e^b)(e^c - e^d) over the receiver
-    // interval [r1, r2] and the source interval [s1, s2], so it equals its
-    // first term times fr fs, fr = 1 - e^{-(r2 - r1) er}, fs = 1 - e^{-(s2 - s1) es}:
-    // six complex exponentials instead of sixteen. With r1 <= r2, s1 <= s2
-    // and Re eta >= 0 the factors have modulus <= 2 and the leading exponent
-    // is the four-term form's first one, so nothing overflows that did not.
+    // CalculateT / CalculateR and the C, D sums: signed sums of four
+    // exponentials e^G (e^a - e^b)(e^c - e^d) over the receiver interval
+    // [r1, r2] and the source interval [s1, s2], each its first term times
+    // fr fs, fr = 1 - e^{-(r2 - r1) er}, fs = 1 - e^{-(s2 - s1) es}. All four
+    // carry the chain's exponentials (chain() below has none).
     double2 Tt, Rr, C = dmk(0, 0), D = dmk(0, 0);
-    const double2 F = lin2(-2 * db1, eb, 2 * dt, et);
-    if (r1 <= r2 && s1 <= s2) {
-        const double2 fsr = dmul(dsub(dmk(1, 0), dexp(dscal(-(r2 - r1), er))),
-                                 dsub(dmk(1, 0), dexp(dscal(-(s2 - s1), es))));
-        Tt = dmul(dexp(lin3(-r1, er, -s1, es, 2 * dt, et)), fsr);
-        Rr = dmul(dexp(lin3(-2 * db1, eb, s2, es, r2, er)), fsr);
-        if (T0.kase == 2) {  // receiver above: CTop, DTop
-            C = dmul(dexp(lin2(-s1, es, r2, er)), fsr);
-            D = dmul(dexp(dadd(dadd(F, dscal(s2, es)), dscal(-r1, er))), fsr);
-        } else if (T0.kase == 1) {  // receiver below: CBot, DBot
-            C = dmul(dexp(lin2(-r1, er, s2, es)), fsr);
-            D = dmul(dexp(dadd(dadd(F, dscal(-s1, es)), dscal(r2, er))), fsr);
+    const double2 *Y = lay + 12L * L * nl;
+    {
+        const long ro = (long)T0.rc * nl + m, so = (long)T0.tr * nl + m, st = (long)nz * nl;
+        const double2 fsr = dmul(dec[ro], dec[so]);
+        const double2 ur = dec[st + ro], us = dec[st + so], dr = dec[2 * st + ro], ds = dec[2 * st + so];
+        const double2 yt = Y[(long)t * nl + m], yb = Y[(long)b * nl + m];
+        Tt = dmul(dmul(ur, us), fsr);
+        Rr = dmul(dmul(dr, ds), fsr);
+        if (T0.kase) {
+            // receiver above (2): CTop, DTop; below (1): CBot, DBot
+            const double2 near = T0.kase == 2 ? dmul(dr, us) : dmul(ur, ds);
+            const double2 far = dmul(T0.kase == 2 ? dmul(ur, ds) : dmul(dr, us), fsr);
+            const double gap = T0.kase == 2 ? T0.s1 - r2 : r1 - T0.s2;
+            C = dmul(r == s ? dexp(dscal(-gap, er)) : near, fsr);
+            D = dmul(yb, far);
         }
-    } else {
-        Tt = dexp(lin3(-r1, er, -s1, es, 2 * dt, et));
-        Tt = dsub(Tt, dexp(lin3(-r1, er, -s2, es, 2 * dt, et)));
-        Tt = dsub(Tt, dexp(lin3(-r2, er, -s1, es, 2 * dt, et)));
-        Tt = dadd(Tt, dexp(lin3(-r2, er, -s2, es, 2 * dt, et)));
-        Rr = dexp(lin3(-2 * db1, eb, s2, es, r2, er));
-        Rr = dsub(Rr, dexp(lin3(-2 * db1, eb, s1, es, r2, er)));
-        Rr = dsub(Rr, dexp(lin3(-2 * db1, eb, s2, es, r1, er)));
-        Rr = dadd(Rr, dexp(lin3(-2 * db1, eb, s1, es, r1, er)));
-        if (T0.kase == 2) {
-            C = dexp(lin2(-s1, es, r2, er));
-            C = dsub(C, dexp(lin2(-s2, es, r2, er)));
-            C = dsub(C, dexp(lin2(-s1, es, r1, er)));
-            C = dadd(C, dexp(lin2(-s2, es, r1, er)));
-            D = dexp(dadd(dadd(F, dscal(s2, es)), dscal(-r1, er)));
-            D = dsub(D, dexp(dadd(dadd(F, dscal(s1, es)), dscal(-r1, er))));
-            D = dsub(D, dexp(dadd(dadd(F, dscal(s2, es)), dscal(-r2, er))));
-            D = dadd(D, dexp(dadd(dadd(F, dscal(s1, es)), dscal(-r2, er))));
-        } else if (T0.kase == 1) {
-            C = dexp(lin2(-r1, er, s2, es));
-            C = dsub(C, dexp(lin2(-r1, er, s1, es)));
-            C = dsub(C, dexp(lin2(-r2, er, s2, es)));
-            C = dadd(C, dexp(lin2(-r2, er, s1, es)));
-            D = dexp(dadd(dadd(F, dscal(-s1, es)), dscal(r2, er)));
-            D = dsub(D, dexp(dadd(dadd(F, dscal(-s2, es)), dscal(r2, er))));
-            D = dsub(D, dexp(dadd(dadd(F, dscal(-s1, es)), dscal(r1, er))));
-            D = dadd(D, dexp(dadd(dadd(F, dscal(-s2, es)), dscal(r1, er))));
+        if (r != s) {
+            Tt = dmul(Tt, yt);
+            Rr = dmul(Rr, yb);
+            D = dmul(D, yt);
         }
     }
-    // propagator chain A[t, b] of a mode from the per-layer pieces of
-    // k_chain_factors
+    // propagator chain A[t, b] of a mode without its exponentials but the
+    // decays across whole layers between t and b
     auto chain = [&](int mode) {
-        const double2 *F = lay + (6L + mode) * L * nl, *H = lay + (8L + mode) * L * nl;
+        const double2 *G = lay + (10L + mode) * L * nl, *H = lay + (8L + mode) * L * nl;
         double2 A = H[(long)b * nl + m];
-        for (int k = b - 1; k >= t; k--) A = dmul(F[(long)k * nl + m], A);
+        for (int k = b - 1; k >= t; k--) {
+            A = dmul(G[(long)k * nl + m], A);
+            if (k > t) A = dmul(Y[(long)k * nl + m], A);
+        }
         return A;
     };
     auto psi1 = [&](const double2 *P, const double2 *Q) {
@@ -286,8 +294,8 @@ __global__ void k_kernels(const double *__restrict__ lam, int nl, const double2 
     const double2 annf = drecip(dmul(er, es));
     const double2 zr2 = dscal(2.0, a.zeta[r]);
     long out = 0;
-    double2 *Ub = U + (long)tr * nl_total + col0 + m;
-    const long ustride = (long)ntrans * nl_total;
+    double2 *Ub = U + (long)tr * nl + m;
+    const long ustride = (long)ntrans * nl;
     if (which & 1) {
         double2 ann = chain(0);
         double2 u = dmul(dmul(ann, annf), special(P1, Q1, 1, 1, psi1(P1, Q1)));
@@ -332,9 +340,11 @@ __global__ void k_kernels(const double *__restrict__ lam, int nl, const double2 
 #undef E
 }
 
-// I[u][trans][g] = norm * sum_j h[430 - j] * U[u][trans][col0 + i + j]
-__global__ void k_hankel(const double2 *__restrict__ U, int nu, int ntrans, long nl_total, long col0, int nrho,
-                         const double *__restrict__ rho, const int *__restrict__ gidx, const int *__restrict__ use_h0,
+// I[u][trans][g] = norm * sum_j h[430 - j] * U[u][trans][col + j], for the
+// radii of all plan items: item radius i has value rho[i], slot g = at[i].x
+// and its first lambda at column at[i].y
+__global__ void k_hankel(const double2 *__restrict__ U, int nu, int ntrans, long nl, int nrho,
+                         const double *__restrict__ rho, const int2 *__restrict__ at, const int *__restrict__ use_h0,
                          const int *__restrict__ negate, double2 *__restrict__ I, int nrad, double den_scale) {
     long idx = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= (long)nu * ntrans * nrho) return;
@@ -342,7 +352,8 @@ __global__ void k_hankel(const double2 *__restrict__ U, int nu, int ntrans, long
     long rest = idx / nrho;
     int tr = (int)(rest % ntrans);
     int u = (int)(rest / ntrans);
-    const double2 *f = U + ((long)u * ntrans + tr) * nl_total + col0 + i;
+    const int2 p = at[i];
+    const double2 *f = U + ((long)u * ntrans + tr) * nl + p.y;
     const double *h = use_h0[u] ? c_h0 : c_h1;
     double sx = 0, sy = 0;
     for (int j = 0; j < kTaps; j++) {
@@ -356,7 +367,7 @@ __global__ void k_hankel(const double2 *__restrict__ U, int nu, int ntrans, long
         sx = -sx;
         sy = -sy;
     }
-    I[((long)u * ntrans + tr) * nrad + gidx[i]] = dmk(sx / den, sy / den);
+    I[((long)u * ntrans + tr) * nrad + p.x] = dmk(sx / den, sy / den);
 }
 
 // IA/IB[u][seg][trans]; with IA32/IB32 also as float pairs {re h, re l,
@@ -829,7 +840,7 @@ __device__ VtpTerms vtp_terms(const double2 *Eta, const double2 *P, const double
 // ("1": the P1/Q1/A1 mode, "s": the sigma mode).
 __global__ void k_kernels_vtp(const double *__restrict__ lam, int nl, const double2 *__restrict__ lay,
                               const LayerArgs a, const Trans *__restrict__ trans, int ntrans, int kind,
-                              double2 *__restrict__ U, long nl_total, long col0) {
+                              double2 *__restrict__ U) {
     long idx = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= (long)ntrans * nl) return;
     const int tr = (int)(idx / nl);
@@ -865,8 +876,8 @@ __global__ void k_kernels_vtp(const double *__restrict__ lam, int nl, const doub
     auto u4 = [&](const double2 *P, const double2 *Q, const VtpTerms &v, double2 A) {
         return dmul(A, dsub(pre(P, Q, v, -1), v.psi34));
     };
-    double2 *Ub = U + (long)tr * nl_total + col0 + m;
-    const long us = (long)ntrans * nl_total;
+    double2 *Ub = U + (long)tr * nl + m;
+    const long us = (long)ntrans * nl;
     if (kind == 0) {
         const double2 zr2 = dscal(2.0, a.zeta[r]);
         Ub[0] = dmul(u1(P1, Q1, v1, a1), dmk(0.0, a.omega * kMu0 * 0.5));
@@ -1140,6 +1151,44 @@ static void load_hankel_taps() {
     loaded.insert(dev);
 }
 
+// The plan's items side by side: all lambdas and radii in one list each, so
+// that every stage is one launch over all of them.
+struct PlanLists {
+    std::vector<double> lam, rho;
+    std::vector<int2> at;  // per item radius: its slot, the column of its first lambda
+    double *d_lam = nullptr, *d_rho = nullptr;
+    int2 *d_at = nullptr;
+    PlanLists(const std::vector<std::vector<double>> &items, const std::vector<std::vector<double>> &lams,
+              const std::vector<std::vector<int>> &gidx, const std::vector<long> &col0) {
+        for (size_t it = 0; it < items.size(); it++) {
+            lam.insert(lam.end(), lams[it].begin(), lams[it].end());
+            rho.insert(rho.end(), items[it].begin(), items[it].end());
+            for (size_t j = 0; j < items[it].size(); j++) at.push_back(make_int2(gidx[it][j], (int)(col0[it] + (long)j)));
+        }
+    }
+    // upload, and the layer recursions of all lambdas
+    void layers(GreenWorkspace &w, const LayerArgs &la, cudaStream_t s, long *launches) {
+        const int nl = (int)lam.size();
+        d_lam = dev_upload(w.d_lam, lam, s);
+        d_rho = dev_upload(w.d_rho, rho, s);
+        d_at = dev_upload(w.d_gidx, at, s);
+        w.d_lay.ensure((size_t)kLayArrays * la.L * nl * sizeof(double2));
+        k_layers<<<dim3((nl + 31) / 32, 2), 32, 0, s>>>(d_lam, nl, la, w.d_lay.as<double2>());
+        k_chain_factors<<<dim3((nl + 127) / 128, la.L), 128, 0, s>>>(nl, la, w.d_lay.as<double2>());
+        EGX_CUDA(cudaGetLastError());
+        if (launches) *launches += 2;
+    }
+    void hankel(GreenWorkspace &w, int nu, int ntrans, const int *use_h0, const int *negate, int nrad, double den,
+                cudaStream_t s, long *launches) {
+        const int nrho = (int)rho.size();
+        const long n = (long)nu * ntrans * nrho;
+        k_hankel<<<(unsigned)((n + 127) / 128), 128, 0, s>>>(w.d_U.as<double2>(), nu, ntrans, (long)lam.size(), nrho,
+                                                             d_rho, d_at, use_h0, negate, w.d_I.as<double2>(), nrad, den);
+        EGX_CUDA(cudaGetLastError());
+        if (launches) *launches += 1;
+    }
+};
+
 void build_green(const GreenModel &m, int n_hankels, cudaStream_t s, DevBuf &quad, GreenBuildStats *stats,
                  long *launches, Timers *tm, GreenWorkspace *ws, bool lateral_fft32) {
     auto t_start = std::chrono::steady_clock::now();
@@ -1220,6 +1269,7 @@ void build_green(const GreenModel &m, int n_hankels, cudaStream_t s, DevBuf &qua
     std::vector<double> bthick(m.bg_thick.begin(), m.bg_thick.end());
     auto make_trans = [&](int rc, int tr) {
         Trans t;
+        t.rc = rc, t.tr = tr;
         t.r1 = m.depth[rc];
         t.r2 = m.depth[rc] + m.thick[rc];
         t.s1 = m.depth[tr];
@@ -1246,9 +1296,9 @@ void build_green(const GreenModel &m, int n_hankels, cudaStream_t s, DevBuf &qua
 
     GreenWorkspace local_ws;
     GreenWorkspace &w = ws ? *ws : local_ws;
-    DevBuf &d_lam = w.d_lam, &d_lay = w.d_lay, &d_trans = w.d_trans, &d_U = w.d_U, &d_I = w.d_I, &d_rho = w.d_rho,
-           &d_gidx = w.d_gidx, &d_flags = w.d_flags, &d_neg = w.d_neg, &d_radii = w.d_radii, &d_IA = w.d_IA,
-           &d_IB = w.d_IB, &d_buf = w.d_buf;
+    DevBuf &d_lay = w.d_lay, &d_trans = w.d_trans, &d_U = w.d_U, &d_I = w.d_I,
+           &d_flags = w.d_flags, &d_neg = w.d_neg, &d_radii = w.d_radii, &d_IA = w.d_IA, &d_IB = w.d_IB,
+           &d_buf = w.d_buf;
     {
         std::vector<double> key = {(double)m.nx, (double)m.ny, m.dx, m.dy};
         key.insert(key.end(), radii.begin(), radii.end());
@@ -1264,6 +1314,13 @@ void build_green(const GreenModel &m, int n_hankels, cudaStream_t s, DevBuf &qua
         if (lateral_fft32) fft_tables32(w, 2 * m.nx, 2 * m.ny, s);
     }
     double *radii_dev = dev_upload(d_radii, radii, s);
+    PlanLists plan(items, lams, gidx, col0);
+    {
+        int ev = tm ? tm->begin(EGX_K_GREEN_LAYERS, s) : -1;
+        plan.layers(w, la, s, launches);
+        if (tm) tm->end(ev, s);
+    }
+    const int nl = (int)nl_total;
 
     // the two halves: asym (U3 -> xz, yz), symm (U1, U2, U5 -> xx, xy, yy, zz)
     for (int half = 0; half < 2; half++) {
@@ -1279,34 +1336,24 @@ void build_green(const GreenModel &m, int n_hankels, cudaStream_t s, DevBuf &qua
         d_I.ensure((size_t)nu * ntrans * nrad * sizeof(double2));
         int *dflags = dev_upload(d_flags, use_h0, s);
         int *dneg = dev_upload(d_neg, negate, s);
-        for (size_t it = 0; it < items.size(); it++) {
-            const int nl = (int)lams[it].size();
-            double *dl = dev_upload(d_lam, lams[it], s);
-            d_lay.ensure((size_t)10 * L * nl * sizeof(double2));
-            int ev = tm ? tm->begin(EGX_K_GREEN_LAYERS, s) : -1;
-            k_layers<<<(nl + 127) / 128, 128, 0, s>>>(dl, nl, la, d_lay.as<double2>());
-            k_chain_factors<<<(nl + 127) / 128, 128, 0, s>>>(nl, la, d_lay.as<double2>());
-            if (launches) *launches += 1;
-            if (tm) tm->end(ev, s);
-            long nthreads = (long)ntrans * nl;
-            ev = tm ? tm->begin(EGX_K_GREEN_KERNELS, s) : -1;
-            k_kernels<<<(unsigned)((nthreads + 127) / 128), 128, 0, s>>>(dl, nl, d_lay.as<double2>(), la, dtrans,
-                                                                          ntrans, which, d_U.as<double2>(), nl_total,
-                                                                          col0[it]);
-            if (tm) tm->end(ev, s);
-            const int nrho = (int)items[it].size();
-            double *drho = dev_upload(d_rho, items[it], s);
-            int *dg = dev_upload(d_gidx, gidx[it], s);
-            long nh_threads = (long)nu * ntrans * nrho;
-            ev = tm ? tm->begin(EGX_K_GREEN_HANKEL, s) : -1;
-            k_hankel<<<(unsigned)((nh_threads + 127) / 128), 128, 0, s>>>(d_U.as<double2>(), nu, ntrans, nl_total,
-                                                                           col0[it], nrho, drho, dg, dflags, dneg,
-                                                                           d_I.as<double2>(), nrad, 2.0 * M_PI);
-            if (tm) tm->end(ev, s);
-            // the per-item uploads above reuse buffers: finish before the next item
-            EGX_CUDA(cudaStreamSynchronize(s));
-            if (launches) *launches += 3;
-        }
+        // the transmitter of each anomaly layer
+        std::vector<int> diag(m.nz);
+        for (int i = 0; i < ntrans; i++)
+            if (tl[i].rc == tl[i].tr) diag[tl[i].tr] = i;
+        int *ddiag = dev_upload(w.d_diag, diag, s);
+        w.d_dec.ensure((size_t)3 * m.nz * nl * sizeof(double2));
+        int ev = tm ? tm->begin(EGX_K_GREEN_KERNELS, s) : -1;
+        k_decays<<<dim3((nl + 127) / 128, m.nz), 128, 0, s>>>(nl, d_lay.as<double2>(), la, dtrans, ddiag, m.nz,
+                                                              w.d_dec.as<double2>());
+        const long nthreads = (long)ntrans * nl;
+        k_kernels<<<(unsigned)((nthreads + 127) / 128), 128, 0, s>>>(plan.d_lam, nl, d_lay.as<double2>(),
+                                                                      w.d_dec.as<double2>(), m.nz, la, dtrans, ntrans,
+                                                                      which, d_U.as<double2>());
+        if (tm) tm->end(ev, s);
+        ev = tm ? tm->begin(EGX_K_GREEN_HANKEL, s) : -1;
+        plan.hankel(w, nu, ntrans, dflags, dneg, nrad, 2.0 * M_PI, s, launches);
+        if (tm) tm->end(ev, s);
+        if (launches) *launches += 2;
         const int nseg = nrad - 1;
         d_IA.ensure((size_t)nu * nseg * ntrans * sizeof(double2));
         d_IB.ensure((size_t)nu * nseg * ntrans * sizeof(double2));
@@ -1505,6 +1552,7 @@ void build_level_green(const GreenModel &m, int n_hankels, double z, double shx,
     std::vector<Trans> tl;
     for (int k = 0; k < m.nz; k++) {
         Trans t;
+        t.rc = t.tr = k;
         t.r1 = t.r2 = z;
         t.s1 = m.depth[k];
         t.s2 = m.depth[k] + m.thick[k];
@@ -1526,25 +1574,15 @@ void build_level_green(const GreenModel &m, int n_hankels, double z, double shx,
     double *radii_dev = dev_upload(w.d_radii, radii, s);
     w.d_U.ensure((size_t)nu * ntrans * nl_total * sizeof(double2));
     w.d_I.ensure((size_t)nu * ntrans * nrad * sizeof(double2));
-    for (size_t it = 0; it < items.size(); it++) {
-        const int nl = (int)lams[it].size();
-        double *dl = dev_upload(w.d_lam, lams[it], s);
-        w.d_lay.ensure((size_t)10 * L * nl * sizeof(double2));
-        k_layers<<<(nl + 127) / 128, 128, 0, s>>>(dl, nl, la, w.d_lay.as<double2>());
-        k_chain_factors<<<(nl + 127) / 128, 128, 0, s>>>(nl, la, w.d_lay.as<double2>());
-        if (launches) *launches += 1;
+    PlanLists plan(items, lams, gidx, col0);
+    plan.layers(w, la, s, launches);
+    {
+        const int nl = (int)nl_total;
         const long nthreads = (long)ntrans * nl;
-        k_kernels_vtp<<<(unsigned)((nthreads + 127) / 128), 128, 0, s>>>(
-            dl, nl, w.d_lay.as<double2>(), la, dtrans, ntrans, kind, w.d_U.as<double2>(), nl_total, col0[it]);
-        const int nrho = (int)items[it].size();
-        double *drho = dev_upload(w.d_rho, items[it], s);
-        int *dg = dev_upload(w.d_gidx, gidx[it], s);
-        const long nh_threads = (long)nu * ntrans * nrho;
-        k_hankel<<<(unsigned)((nh_threads + 127) / 128), 128, 0, s>>>(w.d_U.as<double2>(), nu, ntrans, nl_total,
-                                                                       col0[it], nrho, drho, dg, dflags, dneg,
-                                                                       w.d_I.as<double2>(), nrad, den);
-        EGX_CUDA(cudaStreamSynchronize(s));  // per-item uploads reuse buffers
-        if (launches) *launches += 3;
+        k_kernels_vtp<<<(unsigned)((nthreads + 127) / 128), 128, 0, s>>>(plan.d_lam, nl, w.d_lay.as<double2>(), la, dtrans,
+                                                                          ntrans, kind, w.d_U.as<double2>());
+        plan.hankel(w, nu, ntrans, dflags, dneg, nrad, den, s, launches);
+        if (launches) *launches += 1;
     }
     if (add_zero) {
         const double a2 = step * step;

@@ -31,7 +31,8 @@ struct GreenBuildStats {
 // scratch buffers, and per component the face-integration term lists (CSR),
 // which depend only on the lateral mesh and the radii -- not on frequency.
 struct GreenWorkspace {
-    DevBuf d_lam, d_lay, d_trans, d_U, d_I, d_rho, d_gidx, d_flags, d_neg, d_radii, d_IA, d_IB, d_buf, tw0, tw1;
+    DevBuf d_lam, d_lay, d_dec, d_diag, d_trans, d_U, d_I, d_rho, d_gidx, d_flags, d_neg, d_radii, d_IA, d_IB, d_buf,
+        tw0, tw1;
     DevBuf d_buf32, tw0_32, tw1_32;  // the complex64 lateral FFT of the mixed form
     int n64[2] = {0, 0}, n32[2] = {0, 0};  // lengths of the tables in tw0, tw1 and tw0_32, tw1_32
     DevBuf d_IA32, d_IB32;           // its face-sum coefficients as float pairs

@@ -100,6 +100,18 @@ void make_digits(egx_ctx *ctx, egx_green *g) {
     digitise(g->g64.as<double2>(), g->dig.p, gd, ctx->stream, &ctx->launches);
 }
 
+// the context's scratch of vector sums (on its stream)
+GsScratch sum_scratch(egx_ctx *ctx, int nblocks) {
+    if (!ctx->nrm_counter.p) {
+        ctx->nrm_counter.ensure(sizeof(unsigned));
+        EGX_CUDA(cudaMemsetAsync(ctx->nrm_counter.p, 0, sizeof(unsigned), ctx->stream));
+    }
+    ctx->nrm_part.ensure((size_t)nblocks * 64 * sizeof(double2));
+    GsScratch g;
+    g.partials = ctx->nrm_part.as<double2>(), g.counter = ctx->nrm_counter.as<unsigned>(), g.nblocks = nblocks;
+    return g;
+}
+
 // Forget the captured inner-cycle graph (egx_set_graphs).
 void drop_graph(egx_ctx *ctx) {
     if (ctx->pc_exec) cudaGraphExecDestroy(ctx->pc_exec);
@@ -432,13 +444,12 @@ GmresResult mixed_dev(egx_ctx *ctx, const double2 *b, double2 *x, const egx_mixe
     ctx->mix_t.ensure(N * sizeof(double2));
     ctx->mix_r32.ensure(N * sizeof(float2));
     ctx->mix_d32.ensure(N * sizeof(float2));
-    ctx->nrm_part.ensure(2048 * sizeof(double));
     ctx->nrm_out.ensure(sizeof(double));
     double2 *r = ctx->mix_r.as<double2>(), *t = ctx->mix_t.as<double2>();
     float2 *r32 = ctx->mix_r32.as<float2>(), *d32 = ctx->mix_d32.as<float2>();
     auto norm64 = [&](const double2 *v, long len) {
-        VecOps<double>::norm2(v, len, ctx->nrm_out.as<double>(), ctx->nrm_part.as<double>(), 1024, ctx->stream);
-        ctx->launches += 2;
+        VecOps<double>::norm2(v, len, ctx->nrm_out.as<double>(), sum_scratch(ctx, GsScratch::kMaxBlocks), ctx->stream);
+        ctx->launches += 1;
         double h;
         EGX_CUDA(cudaMemcpyAsync(&h, ctx->nrm_out.p, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
         EGX_CUDA(cudaStreamSynchronize(ctx->stream));
@@ -1111,12 +1122,10 @@ int egx_dot_products(egx_ctx *ctx, const double *V, int ncols, const double *w, 
             dV = stage;
             dw = stage + (size_t)ncols * n;
         }
-        int nblocks = (int)std::min<long>(1024, (n + 255) / 256);
-        ctx->nrm_part.ensure((size_t)nblocks * 64 * sizeof(double2));
+        int nblocks = (int)std::min<long>(GsScratch::kMaxBlocks, (n + 255) / 256);
         ctx->yout.ensure(64 * sizeof(double2));
-        VecOps<double>::multi_dot(dV, ncols, dw, n, ctx->yout.as<double2>(), ctx->nrm_part.as<double2>(), nblocks,
-                                  ctx->stream);
-        ctx->launches += 2;
+        VecOps<double>::multi_dot(dV, ncols, dw, n, ctx->yout.as<double2>(), sum_scratch(ctx, nblocks), ctx->stream);
+        ctx->launches += 1;
         cudaMemcpyKind k = where == EGX_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost;
         EGX_CUDA(cudaMemcpyAsync(out, ctx->yout.p, ncols * sizeof(double2), k, ctx->stream));
         EGX_CUDA(cudaStreamSynchronize(ctx->stream));

@@ -69,7 +69,7 @@ struct egx_ctx {
     cudaGraphExec_t pc_exec = nullptr;
     std::string pc_key;
     long pc_nodes = 0, pc_replays = 0;
-    egx::DevBuf nrm_part, nrm_out, mix_r, mix_t, mix_r32, mix_d32;
+    egx::DevBuf nrm_part, nrm_counter, nrm_out, mix_r, mix_t, mix_r32, mix_d32;
     egx::DevBuf js, chi0;
     egx::DevBuf errflag;  // device int: EGX_ERR_TIMEOUT from a bounded wait
     egx::GreenBuildStats last_build;

@@ -1,4 +1,5 @@
 // Device vector kernels and the host-side GMRES driver (see egx_krylov.cuh).
+#include <algorithm>
 #include <cmath>
 #include <cstdint>
 
@@ -52,21 +53,105 @@ __device__ double block_sum(double v) {
     return v;
 }
 
+// Sums of NV values over a warp's lanes (NV 16 or 32), each as warp_sum adds
+// them: a lane ends with the sum of value lane / (32 / NV). At each step a
+// lane passes on the half of its values that the other one keeps, so a value
+// costs NV adds a lane instead of five per value; a shuffle tree per value
+// had the FP64 pipes as its bound.
+template <int NV>
+__device__ __forceinline__ double warp_sums(double *v, int lane) {
+    int o = 16;
+#pragma unroll
+    for (int half = NV / 2; half >= 1; half >>= 1, o >>= 1) {
+        const bool up = lane & o;
+#pragma unroll
+        for (int i = 0; i < half; i++) {
+            const double send = up ? v[i] : v[i + half];
+            const double keep = up ? v[i + half] : v[i];
+            v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        }
+    }
+    for (; o > 0; o >>= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+    return v[0];
+}
+
+// whether this block is the last of the grid to get here; what every block
+// wrote before is visible to the last one. The counter is 0 again afterwards.
+__device__ __forceinline__ bool last_block(unsigned *counter) {
+    __shared__ bool last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicInc(counter, gridDim.x - 1) == gridDim.x - 1;
+    __syncthreads();
+    if (last) __threadfence();
+    return last;
+}
+
+// A block's sums of kc columns into the partials, and in the last block to
+// get there the columns' sums over the blocks into out (256 threads). One
+// barrier per chunk of columns: red is double-buffered by `flip`.
+template <int COLS>
+__device__ __forceinline__ void store_partials(const double *acc, int kc, double2 *partials, int flip) {
+    __shared__ double red[2][8][2 * COLS];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    double v[2 * COLS];
+#pragma unroll
+    for (int i = 0; i < 2 * COLS; i++) v[i] = acc[i];
+    const double sum = warp_sums<2 * COLS>(v, lane);
+    constexpr int per = 32 / (2 * COLS);
+    if (lane % per == 0) red[flip][warp][lane / per] = sum;
+    __syncthreads();
+    const int i = threadIdx.x;
+    if (i < 2 * kc) {
+        const double(*r)[2 * COLS] = red[flip];
+        reinterpret_cast<double *>(partials)[i] =
+            ((r[0][i] + r[4][i]) + (r[2][i] + r[6][i])) + ((r[1][i] + r[5][i]) + (r[3][i] + r[7][i]));
+    }
+}
+
+__device__ __forceinline__ void finish_dots(const double2 *partials, int ncols, double2 *out) {
+    const int lane = threadIdx.x & 31, nblocks = (int)gridDim.x;
+    for (int k = threadIdx.x >> 5; k < ncols; k += 8) {
+        // the sums of eight warps of 32 threads, thread t taking blocks t, t + 256, ...
+        double v[16];
+#pragma unroll
+        for (int w = 0; w < 8; w++) {
+            double2 s = make_double2(0, 0);
+            for (int b = 32 * w + lane; b < nblocks; b += 256) {
+                const double2 p = __ldcg(partials + (long)b * ncols + k);
+                s.x += p.x;
+                s.y += p.y;
+            }
+            v[2 * w] = s.x, v[2 * w + 1] = s.y;
+        }
+        double t = warp_sums<16>(v, lane);  // lane 4 w + 2 (component)
+        for (int o = 16; o >= 4; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+        if (lane == 0) out[k].x = t;
+        if (lane == 2) out[k].y = t;
+    }
+}
+
 // Each thread keeps the partial sums of up to kDotCols columns in
 // registers, so w is read once per kDotCols columns (the stacked vectors are
 // larger than L2), and reads DotRows<T> rows per pass, so that enough loads
 // are in flight: eight rows reached 4.2-4.6 TB/s for 1-30 complex64 columns
-// where two rows reached 2.5-3.7.
+// where two rows reached 2.5-3.7. The last block adds up the blocks' sums.
+// `count` (may be null) goes up by one. With their sums by halving exchanges
+// (warp_sums), 445,500 complex64 entries and 10 columns on average: 23 us with
+// the columns' sums, against 36 + 4 with a shuffle tree per value, two
+// barriers per column and a launch for the columns' sums.
 constexpr int kDotCols = 16;
 template <typename T> struct DotRows { static constexpr int value = 8; };
 template <> struct DotRows<double> { static constexpr int value = 4; };
 template <typename T>
 __global__ void k_multi_dot(const C<T> *__restrict__ V, int ncols, const C<T> *__restrict__ w, long n,
-                            double2 *__restrict__ partials, const int *live) {
+                            double2 *partials, double2 *__restrict__ out, unsigned *counter, const int *live,
+                            long long *count) {
     if (live && !*live) return;
+    if (count && blockIdx.x == 0 && threadIdx.x == 0) ++*count;
     constexpr int ROWS = DotRows<T>::value;
     const long stride = (long)gridDim.x * blockDim.x;
-    for (int k0 = 0; k0 < ncols; k0 += kDotCols) {
+    for (int k0 = 0, flip = 0; k0 < ncols; k0 += kDotCols, flip ^= 1) {
         const int kc = min(kDotCols, ncols - k0);
         const C<T> *col = V + (long)k0 * n;
         C<T> acc[kDotCols];
@@ -93,22 +178,22 @@ __global__ void k_multi_dot(const C<T> *__restrict__ V, int ncols, const C<T> *_
             for (int j = 0; j < kDotCols; j++)
                 if (j < kc) cfma_conj<T>(acc[j], col[(long)j * n + r], x);
         }
+        double v[2 * kDotCols];
 #pragma unroll
-        for (int j = 0; j < kDotCols; j++) {
-            if (j < kc) {  // kc is the same in every thread: the block sums stay uniform
-                double2 s = block_sum2(make_double2((double)acc[j].x, (double)acc[j].y));
-                if (threadIdx.x == 0) partials[(long)blockIdx.x * ncols + k0 + j] = s;
-            }
-        }
+        for (int j = 0; j < kDotCols; j++) v[2 * j] = (double)acc[j].x, v[2 * j + 1] = (double)acc[j].y;
+        store_partials<kDotCols>(v, kc, partials + (long)blockIdx.x * ncols + k0, flip);
     }
+    if (last_block(counter)) finish_dots(partials, ncols, out);
 }
 
 // complex64 vectors of even length: the same dots with each load a float4
 // (two complex entries), four per column and pass, eight columns per pass
 // (66 registers: three CTAs per SM where sixteen columns allowed two)
 __global__ void k_multi_dot_c2(const float4 *__restrict__ V, int ncols, const float4 *__restrict__ w, long n2,
-                               double2 *__restrict__ partials, const int *live) {
+                               double2 *partials, double2 *__restrict__ out, unsigned *counter, const int *live,
+                               long long *count) {
     if (live && !*live) return;
+    if (count && blockIdx.x == 0 && threadIdx.x == 0) ++*count;
     constexpr int ROWS = 4, kDotCols = 8;
     const long stride = (long)gridDim.x * blockDim.x;
     auto fma_conj2 = [](float2 &acc, float4 a, float4 b) {  // += conj(a) b, two entries
@@ -121,7 +206,7 @@ __global__ void k_multi_dot_c2(const float4 *__restrict__ V, int ncols, const fl
         acc.y = fmaf(a.z, b.w, acc.y);
         acc.y = fmaf(-a.w, b.z, acc.y);
     };
-    for (int k0 = 0; k0 < ncols; k0 += kDotCols) {
+    for (int k0 = 0, flip = 0; k0 < ncols; k0 += kDotCols, flip ^= 1) {
         const int kc = min(kDotCols, ncols - k0);
         const float4 *col = V + (long)k0 * n2;
         float2 acc[kDotCols];
@@ -148,43 +233,153 @@ __global__ void k_multi_dot_c2(const float4 *__restrict__ V, int ncols, const fl
             for (int j = 0; j < kDotCols; j++)
                 if (j < kc) fma_conj2(acc[j], col[(long)j * n2 + r], x);
         }
+        double v[2 * kDotCols];
 #pragma unroll
-        for (int j = 0; j < kDotCols; j++) {
-            if (j < kc) {
-                double2 sm = block_sum2(make_double2((double)acc[j].x, (double)acc[j].y));
-                if (threadIdx.x == 0) partials[(long)blockIdx.x * ncols + k0 + j] = sm;
-            }
+        for (int j = 0; j < kDotCols; j++) v[2 * j] = (double)acc[j].x, v[2 * j + 1] = (double)acc[j].y;
+        store_partials<kDotCols>(v, kc, partials + (long)blockIdx.x * ncols + k0, flip);
+    }
+    if (last_block(counter)) finish_dots(partials, ncols, out);
+}
+
+// a block's squared norms into the partials, and in the last block their sum
+// into *out; true there
+__device__ __forceinline__ bool finish_norm(double acc, double *partials, double *out, unsigned *counter) {
+    const double s = block_sum(acc);
+    if (threadIdx.x == 0) partials[blockIdx.x] = s;
+    if (!last_block(counter)) return false;
+    double t = 0;
+    for (int b = threadIdx.x; b < (int)gridDim.x; b += blockDim.x) t += __ldcg(partials + b);
+    t = block_sum(t);
+    if (threadIdx.x == 0) *out = t;
+    return true;
+}
+
+// ------------------------------------------------------------ device control
+//
+// Device code that takes the host's decisions of GmresSolver
+// (Extreme.Fgmres/Gmres.cs:77-348) on the device state GmState: the
+// right-hand side and initial residual norms (:80-107), the classical
+// Gram-Schmidt pass bookkeeping and its re-orthogonalisation test
+// (:252-262, :297-313), the Givens rotations and the Arnoldi backward error
+// (:271-292), and the upper-triangular solve of the solution update
+// (:187-196, SimplifiedZtrsv). The arithmetic is the host driver's, in the
+// same order; complex moduli and quotients use hypot and Smith's division.
+
+__device__ __forceinline__ double cabs2(double2 a) { return hypot(a.x, a.y); }
+__device__ __forceinline__ double2 cmul2(double2 a, double2 b) {
+    return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
+}
+__device__ __forceinline__ double2 cconj2(double2 a) { return make_double2(a.x, -a.y); }
+// x, y <- c x + s y, c y - conj(s) x (zrot)
+__device__ __forceinline__ void zrot_dev(double2 &x, double2 &y, double c, double2 s) {
+    const double2 sy = cmul2(s, y), sx = cmul2(cconj2(s), x);
+    const double2 t = make_double2(c * x.x + sy.x, c * x.y + sy.y);
+    y = make_double2(c * y.x - sx.x, c * y.y - sx.y);
+    x = t;
+}
+
+// Control of a Gram-Schmidt pass, in the last block of its update kernel: st
+// null, none.
+struct GsControl {
+    GmState *st;
+    double2 *H;
+    double *cs;
+    double2 *sn;
+    int j, m, pass, max_pass;
+    double tol;
+
+    // the pass's bookkeeping (h(0..j, j) += dots, dloo, ||w|| and the
+    // re-orthogonalisation test 2 ||w|| <= sqrt(dloo)); after the last pass
+    // the rest of the step
+    __device__ void finish(const double2 *dots, const double *norm2) const {
+        if (!st) return;
+        double2 *h = H + (size_t)j * (m + 1);
+        for (int i = threadIdx.x; i <= j; i += blockDim.x) {
+            const double2 d = dots[i];
+            const double2 o = pass == 1 ? make_double2(0.0, 0.0) : h[i];
+            h[i] = make_double2(o.x + d.x, o.y + d.y);
         }
+        if (threadIdx.x == 0) {
+            double ss = 0;
+#pragma unroll 4
+            for (int i = 0; i <= j; i++) {
+                const double2 d = dots[i];
+                ss += d.x * d.x + d.y * d.y;
+            }
+            st->dloo = ss;
+            st->dnormw = sqrt(*norm2);
+            st->reorth = (2.0 * st->dnormw <= sqrt(ss) && pass < max_pass) ? 1 : 0;
+        }
+        __syncthreads();
+        if (pass == max_pass) step();
     }
-}
 
-__global__ void k_reduce_cols(const double2 *__restrict__ partials, int nblocks, int ncols, double2 *__restrict__ out,
-                              const int *live) {
-    if (live && !*live) return;
-    const int k = blockIdx.x;
-    double2 s = make_double2(0, 0);
-    for (int b = threadIdx.x; b < nblocks; b += blockDim.x) {
-        double2 p = partials[(long)b * ncols + k];
-        s.x += p.x;
-        s.y += p.y;
+    // a pass that the previous one did not ask for: the rest of the step all
+    // the same if it is the last
+    __device__ void skipped() const {
+        if (st && pass == max_pass && blockIdx.x == 0 && st->active) step();
     }
-    s = block_sum2(s);
-    if (threadIdx.x == 0) out[k] = s;
-}
 
-__global__ void k_reduce_scalar(const double *__restrict__ partials, int nblocks, double *__restrict__ out,
-                                const int *live) {
-    if (live && !*live) return;
-    double s = 0;
-    for (int b = threadIdx.x; b < nblocks; b += blockDim.x) s += partials[b];
-    s = block_sum(s);
-    if (threadIdx.x == 0) out[0] = s;
-}
-
+    // the rest of step j: h(j+1, j) = ||w||, the previous rotations, zrotg,
+    // the rotation of the rhs column, bea = |g_{j+1}| / ||b||; the cycle stops
+    // when bea <= tol, after m steps, or on a non-finite bea. One thread's
+    // recurrence, its operands in shared memory (from global memory it waited
+    // 13 us on loads at 20 columns).
+    __device__ void step() const {
+        __shared__ double2 h[64], s_sn[64];
+        __shared__ double s_cs[64];
+        double2 *hg = H + (size_t)j * (m + 1);
+        double2 *g = H + (size_t)m * (m + 1);
+        for (int i = threadIdx.x; i <= j; i += blockDim.x) {
+            h[i] = hg[i];
+            if (i < j) s_cs[i] = cs[i], s_sn[i] = sn[i];
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            h[j + 1] = make_double2(st->dnormw, 0.0);
+            for (int i = 0; i < j; i++) zrot_dev(h[i], h[i + 1], s_cs[i], s_sn[i]);
+            double c;
+            double2 sv;
+            {  // zrotg (classic reference algorithm)
+                const double2 a = h[j], b = h[j + 1];
+                const double aa = cabs2(a);
+                if (aa == 0.0) {
+                    c = 0.0;
+                    sv = make_double2(1.0, 0.0);
+                } else {
+                    const double scale = aa + cabs2(b);
+                    const double a1 = cabs2(make_double2(a.x / scale, a.y / scale));
+                    const double b1 = cabs2(make_double2(b.x / scale, b.y / scale));
+                    const double nrm = scale * sqrt(a1 * a1 + b1 * b1);
+                    const double2 alpha = make_double2(a.x / aa, a.y / aa);
+                    c = aa / nrm;
+                    const double2 t = cmul2(alpha, cconj2(b));
+                    sv = make_double2(t.x / nrm, t.y / nrm);
+                }
+                cs[j] = c;
+                sn[j] = sv;
+            }
+            zrot_dev(g[j], g[j + 1], c, sv);
+            zrot_dev(h[j], h[j + 1], c, sv);
+            h[j + 1] = make_double2(0.0, 0.0);
+            const double bea = cabs2(g[j + 1]) / st->bn;
+            st->bea = bea;
+            st->iterations++;
+            st->jh = j + 1;
+            if (!isfinite(bea)) st->flags |= kGmNonFinite;
+            if (!(bea > tol && j + 1 < m)) st->active = 0;
+        }
+        __syncthreads();
+        for (int i = threadIdx.x; i <= j + 1; i += blockDim.x) hg[i] = h[i];
+    }
+};
 template <typename T>
 __global__ void k_update_norm(const C<T> *__restrict__ V, int ncols, const double2 *__restrict__ dots, C<T> *w, long n,
-                              double *__restrict__ partials, const int *live) {
-    if (live && !*live) return;
+                              double *partials, double *out, unsigned *counter, const int *live, const GsControl gs) {
+    if (live && !*live) {
+        gs.skipped();
+        return;
+    }
     __shared__ C<T> sd[64];
     for (int k = threadIdx.x; k < ncols; k += blockDim.x) sd[k] = mk<T>((T)dots[k].x, (T)dots[k].y);
     __syncthreads();
@@ -205,14 +400,17 @@ __global__ void k_update_norm(const C<T> *__restrict__ V, int ncols, const doubl
         acc = fma(v.x, v.x, acc);
         acc = fma(v.y, v.y, acc);
     }
-    double s = block_sum((double)acc);
-    if (threadIdx.x == 0) partials[blockIdx.x] = s;
+    if (finish_norm((double)acc, partials, out, counter)) gs.finish(dots, out);
 }
 
 // complex64 vectors of even length: the update with float4 loads
 __global__ void k_update_norm_c2(const float4 *__restrict__ V, int ncols, const double2 *__restrict__ dots, float4 *w,
-                                 long n2, double *__restrict__ partials, const int *live) {
-    if (live && !*live) return;
+                                 long n2, double *partials, double *out, unsigned *counter, const int *live,
+                                 const GsControl gs) {
+    if (live && !*live) {
+        gs.skipped();
+        return;
+    }
     __shared__ float2 sd[64];
     for (int k = threadIdx.x; k < ncols; k += blockDim.x) sd[k] = make_float2((float)dots[k].x, (float)dots[k].y);
     __syncthreads();
@@ -239,12 +437,12 @@ __global__ void k_update_norm_c2(const float4 *__restrict__ V, int ncols, const 
         acc = fmaf(v.z, v.z, acc);
         acc = fmaf(v.w, v.w, acc);
     }
-    double sm = block_sum((double)acc);
-    if (threadIdx.x == 0) partials[blockIdx.x] = sm;
+    if (finish_norm((double)acc, partials, out, counter)) gs.finish(dots, out);
 }
 
 template <typename T>
-__global__ void k_norm2(const C<T> *__restrict__ x, long n, double *__restrict__ partials, const int *live) {
+__global__ void k_norm2(const C<T> *__restrict__ x, long n, double *partials, double *out, unsigned *counter,
+                        const int *live) {
     if (live && !*live) return;
     const long stride = (long)gridDim.x * blockDim.x;
     T acc = 0;
@@ -253,8 +451,7 @@ __global__ void k_norm2(const C<T> *__restrict__ x, long n, double *__restrict__
         acc = fma(v.x, v.x, acc);
         acc = fma(v.y, v.y, acc);
     }
-    double s = block_sum((double)acc);
-    if (threadIdx.x == 0) partials[blockIdx.x] = s;
+    finish_norm((double)acc, partials, out, counter);
 }
 
 template <typename T>
@@ -283,14 +480,8 @@ __global__ void k_sub(const C<T> *__restrict__ a, const C<T> *__restrict__ b, C<
         y[r] = csub<T>(a[r], b[r]);
 }
 template <typename T>
-__global__ void k_add(const C<T> *__restrict__ x, C<T> *__restrict__ y, long n, const int *live) {
-    if (live && !*live) return;
-    for (long r = (long)blockIdx.x * blockDim.x + threadIdx.x; r < n; r += (long)gridDim.x * blockDim.x)
-        y[r] = cadd<T>(y[r], x[r]);
-}
-template <typename T>
-__global__ void k_gemv(const C<T> *__restrict__ V, int ncols, const double2 *__restrict__ coef, C<T> *__restrict__ out,
-                       long n, const int *ncols_dev) {
+__global__ void k_gemv_add(const C<T> *__restrict__ V, int ncols, const double2 *__restrict__ coef, C<T> *__restrict__ y,
+                           long n, const int *ncols_dev) {
     if (ncols_dev) ncols = *ncols_dev;
     if (ncols <= 0) return;
     __shared__ C<T> sc[64];
@@ -299,7 +490,7 @@ __global__ void k_gemv(const C<T> *__restrict__ V, int ncols, const double2 *__r
     for (long r = (long)blockIdx.x * blockDim.x + threadIdx.x; r < n; r += (long)gridDim.x * blockDim.x) {
         C<T> acc = mk<T>(0, 0);
         for (int k = 0; k < ncols; k++) cfma<T>(acc, V[(long)k * n + r], sc[k]);
-        out[r] = acc;
+        y[r] = cadd<T>(y[r], acc);
     }
 }
 
@@ -326,30 +517,34 @@ static int grid_for(long n) {
 }
 
 template <typename T>
-void VecOps<T>::multi_dot(const C<T> *V, int ncols, const C<T> *w, long n, double2 *dots_dev, double2 *partials,
-                          int nblocks, cudaStream_t s, const int *live) {
+void VecOps<T>::multi_dot(const C<T> *V, int ncols, const C<T> *w, long n, double2 *dots_dev, const GsScratch &g,
+                          cudaStream_t s, const int *live, long long *count) {
     if (sizeof(T) == sizeof(float) && n % 2 == 0 && aligned16(V) && aligned16(w))
-        k_multi_dot_c2<<<nblocks, kThreads, 0, s>>>(reinterpret_cast<const float4 *>(V), ncols,
-                                                    reinterpret_cast<const float4 *>(w), n / 2, partials, live);
+        k_multi_dot_c2<<<g.nblocks, kThreads, 0, s>>>(reinterpret_cast<const float4 *>(V), ncols,
+                                                      reinterpret_cast<const float4 *>(w), n / 2, g.partials, dots_dev,
+                                                      g.counter, live, count);
     else
-        k_multi_dot<T><<<nblocks, kThreads, 0, s>>>(V, ncols, w, n, partials, live);
-    k_reduce_cols<<<ncols, kThreads, 0, s>>>(partials, nblocks, ncols, dots_dev, live);
+        k_multi_dot<T><<<g.nblocks, kThreads, 0, s>>>(V, ncols, w, n, g.partials, dots_dev, g.counter, live, count);
+}
+template <typename T>
+static void launch_update(const C<T> *V, int ncols, const double2 *dots_dev, C<T> *w, long n, double *norm2_dev,
+                          const GsScratch &g, cudaStream_t s, const int *live, const GsControl &gs) {
+    double *part = reinterpret_cast<double *>(g.partials);
+    if (sizeof(T) == sizeof(float) && n % 2 == 0 && aligned16(V) && aligned16(w))
+        k_update_norm_c2<<<g.nblocks, kThreads, 0, s>>>(reinterpret_cast<const float4 *>(V), ncols, dots_dev,
+                                                        reinterpret_cast<float4 *>(w), n / 2, part, norm2_dev,
+                                                        g.counter, live, gs);
+    else
+        k_update_norm<T><<<g.nblocks, kThreads, 0, s>>>(V, ncols, dots_dev, w, n, part, norm2_dev, g.counter, live, gs);
 }
 template <typename T>
 void VecOps<T>::update_norm(const C<T> *V, int ncols, const double2 *dots_dev, C<T> *w, long n, double *norm2_dev,
-                            double *partials, int nblocks, cudaStream_t s, const int *live) {
-    if (sizeof(T) == sizeof(float) && n % 2 == 0 && aligned16(V) && aligned16(w))
-        k_update_norm_c2<<<nblocks, kThreads, 0, s>>>(reinterpret_cast<const float4 *>(V), ncols, dots_dev,
-                                                      reinterpret_cast<float4 *>(w), n / 2, partials, live);
-    else
-        k_update_norm<T><<<nblocks, kThreads, 0, s>>>(V, ncols, dots_dev, w, n, partials, live);
-    k_reduce_scalar<<<1, kThreads, 0, s>>>(partials, nblocks, norm2_dev, live);
+                            const GsScratch &g, cudaStream_t s) {
+    launch_update<T>(V, ncols, dots_dev, w, n, norm2_dev, g, s, nullptr, GsControl{});
 }
 template <typename T>
-void VecOps<T>::norm2(const C<T> *x, long n, double *norm2_dev, double *partials, int nblocks, cudaStream_t s,
-                      const int *live) {
-    k_norm2<T><<<nblocks, kThreads, 0, s>>>(x, n, partials, live);
-    k_reduce_scalar<<<1, kThreads, 0, s>>>(partials, nblocks, norm2_dev, live);
+void VecOps<T>::norm2(const C<T> *x, long n, double *norm2_dev, const GsScratch &g, cudaStream_t s, const int *live) {
+    k_norm2<T><<<g.nblocks, kThreads, 0, s>>>(x, n, reinterpret_cast<double *>(g.partials), norm2_dev, g.counter, live);
 }
 template <typename T>
 void VecOps<T>::scale(const C<T> *x, double a, C<T> *y, long n, cudaStream_t s) {
@@ -368,13 +563,9 @@ void VecOps<T>::sub(const C<T> *a, const C<T> *b, C<T> *y, long n, cudaStream_t 
     k_sub<T><<<grid_for(n), kThreads, 0, s>>>(a, b, y, n, live);
 }
 template <typename T>
-void VecOps<T>::add(const C<T> *x, C<T> *y, long n, cudaStream_t s, const int *live) {
-    k_add<T><<<grid_for(n), kThreads, 0, s>>>(x, y, n, live);
-}
-template <typename T>
-void VecOps<T>::gemv(const C<T> *V, int ncols, const double2 *coef, C<T> *out, long n, cudaStream_t s,
-                     const int *ncols_dev) {
-    k_gemv<T><<<grid_for(n), kThreads, 0, s>>>(V, ncols, coef, out, n, ncols_dev);
+void VecOps<T>::gemv_add(const C<T> *V, int ncols, const double2 *coef, C<T> *y, long n, cudaStream_t s,
+                         const int *ncols_dev) {
+    k_gemv_add<T><<<grid_for(n), kThreads, 0, s>>>(V, ncols, coef, y, n, ncols_dev);
 }
 template <typename T>
 void VecOps<T>::copy(const C<T> *x, C<T> *y, long n, cudaStream_t s) {
@@ -401,8 +592,7 @@ template <typename T>
 Gmres<T>::Gmres(long n, int m, double tol, int max_restarts, bool check_true, cudaStream_t s)
     : n_(n), m_(m), tol_(tol), max_restarts_(max_restarts), check_true_(check_true), s_(s) {
     EGX_CHECK(m >= 1 && m <= 60, EGX_ERR_INVALID, "GMRES buffer length must be in [1, 60]");
-    nblocks_ = grid_for(n);
-    if (nblocks_ > 1024) nblocks_ = 1024;
+    scratch_.nblocks = std::min(grid_for(n), GsScratch::kMaxBlocks);
     auto alloc = [](void **p, size_t b) { *p = device_alloc(b, "GMRES workspace"); };
     alloc((void **)&V_, sizeof(C<T>) * n * m);
     alloc((void **)&w_, sizeof(C<T>) * n);
@@ -411,7 +601,9 @@ Gmres<T>::Gmres(long n, int m, double tol, int max_restarts, bool check_true, cu
     alloc((void **)&dots_, sizeof(double2) * 64 + sizeof(double) * 2);
     norm_dev_ = reinterpret_cast<double *>(dots_ + 64);
     alloc((void **)&coef_, sizeof(double2) * 64);
-    alloc((void **)&partials_, sizeof(double2) * (size_t)nblocks_ * 64);
+    alloc((void **)&scratch_.partials, sizeof(double2) * (size_t)scratch_.nblocks * 64 + sizeof(unsigned));
+    scratch_.counter = reinterpret_cast<unsigned *>(scratch_.partials + (size_t)scratch_.nblocks * 64);
+    EGX_CUDA(cudaMemsetAsync(scratch_.counter, 0, sizeof(unsigned), s));
     EGX_CUDA(cudaMallocHost((void **)&host_, sizeof(double2) * 64 + sizeof(double) * 2));
     alloc((void **)&st_, sizeof(GmState));
     alloc((void **)&napp_dev_, sizeof(long long));
@@ -434,7 +626,7 @@ Gmres<T>::~Gmres() {
     cudaFree(xcur_);
     cudaFree(dots_);
     cudaFree(coef_);
-    cudaFree(partials_);
+    cudaFree(scratch_.partials);
     cudaFree(st_);
     cudaFree(napp_dev_);
     cudaFree(Hd_);
@@ -446,8 +638,8 @@ Gmres<T>::~Gmres() {
 
 template <typename T>
 double Gmres<T>::norm(const C<T> *x) {
-    VecOps<T>::norm2(x, n_, norm_dev_, reinterpret_cast<double *>(partials_), nblocks_, s_);
-    kernel_launches += 2;
+    VecOps<T>::norm2(x, n_, norm_dev_, scratch_, s_);
+    kernel_launches += 1;
     EGX_CUDA(cudaMemcpyAsync(host_, norm_dev_, sizeof(double), cudaMemcpyDeviceToHost, s_));
     EGX_CUDA(cudaStreamSynchronize(s_));
     return std::sqrt(host_[0]);
@@ -467,9 +659,8 @@ void Gmres<T>::construct(int jh, C<T> *result) {
     }
     if (jh > 0) {
         EGX_CUDA(cudaMemcpyAsync(coef_, y.data(), sizeof(double2) * jh, cudaMemcpyHostToDevice, s_));
-        VecOps<T>::gemv(precond ? Z_ : V_, jh, coef_, r0_, n_, s_);
-        VecOps<T>::add(r0_, result, n_, s_);
-        kernel_launches += 2;
+        VecOps<T>::gemv_add(precond ? Z_ : V_, jh, coef_, result, n_, s_);
+        kernel_launches += 1;
         // the host vector y must outlive the async copy
         EGX_CUDA(cudaStreamSynchronize(s_));
     }
@@ -508,13 +699,12 @@ double Gmres<T>::arnoldi(double bn, int &jh) {
             northo++;
             const int koff = sizeof(T) == sizeof(double) ? 0 : EGX_K_C64;
             int ev = timers ? timers->begin(EGX_K_GS_DOTS + koff, s_) : -1;
-            VecOps<T>::multi_dot(V_, jh + 1, w_, n_, dots_, partials_, nblocks_, s_);
+            VecOps<T>::multi_dot(V_, jh + 1, w_, n_, dots_, scratch_, s_);
             if (timers) timers->end(ev, s_);
             ev = timers ? timers->begin(EGX_K_GS_UPDATE + koff, s_) : -1;
-            VecOps<T>::update_norm(V_, jh + 1, dots_, w_, n_, norm_dev_, reinterpret_cast<double *>(partials_),
-                                   nblocks_, s_);
+            VecOps<T>::update_norm(V_, jh + 1, dots_, w_, n_, norm_dev_, scratch_, s_);
             if (timers) timers->end(ev, s_);
-            kernel_launches += 4;
+            kernel_launches += 2;
             EGX_CUDA(cudaMemcpyAsync(host_, dots_, sizeof(double2) * 64 + sizeof(double), cudaMemcpyDeviceToHost, s_));
             EGX_CUDA(cudaStreamSynchronize(s_));
             const double2 *hd = reinterpret_cast<const double2 *>(host_);
@@ -652,30 +842,6 @@ GmresResult Gmres<T>::solve_host(const C<T> *rhs, const C<T> *x0, C<T> *result) 
     return res;
 }
 
-// ------------------------------------------------------------ device control
-//
-// One-thread kernels that take the host's decisions of GmresSolver
-// (Extreme.Fgmres/Gmres.cs:77-348) on the device state GmState: the
-// right-hand side and initial residual norms (:80-107), the classical
-// Gram-Schmidt pass bookkeeping and its re-orthogonalisation test
-// (:252-262, :297-313), the Givens rotations and the Arnoldi backward error
-// (:271-292), and the upper-triangular solve of the solution update
-// (:187-196, SimplifiedZtrsv). The arithmetic is the host driver's, in the
-// same order; complex moduli and quotients use hypot and Smith's division.
-
-__device__ __forceinline__ double cabs2(double2 a) { return hypot(a.x, a.y); }
-__device__ __forceinline__ double2 cmul2(double2 a, double2 b) {
-    return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
-}
-__device__ __forceinline__ double2 cconj2(double2 a) { return make_double2(a.x, -a.y); }
-// x, y <- c x + s y, c y - conj(s) x (zrot)
-__device__ __forceinline__ void zrot_dev(double2 &x, double2 &y, double c, double2 s) {
-    const double2 sy = cmul2(s, y), sx = cmul2(cconj2(s), x);
-    const double2 t = make_double2(c * x.x + sy.x, c * x.y + sy.y);
-    y = make_double2(c * y.x - sx.x, c * y.y - sx.y);
-    x = t;
-}
-
 // a fresh solve: ||rhs|| from its squared norm
 __global__ void k_gm_start(GmState *st, const double *norm2) {
     GmState g;
@@ -713,84 +879,33 @@ __global__ void k_gm_cycle(GmState *st, double2 *H, int m) {
     if (threadIdx.x == 0) st->jh = 0;
 }
 
-// one Gram-Schmidt pass of step j (pass 1: while active; later passes:
-// while the previous one asked for another): h(0..j, j) += dots, dloo,
-// ||w|| and the re-orthogonalisation test 2 ||w|| <= sqrt(dloo)
-__global__ void k_gm_ortho(GmState *st, double2 *H, const double2 *dots, const double *norm2, int j, int m,
-                           int pass, int max_pass) {
-    if (!(pass == 1 ? st->active : st->reorth)) return;
-    double2 *h = H + (size_t)j * (m + 1);
-    double ss = 0;
-    for (int i = 0; i <= j; i++) {
-        const double2 d = dots[i];
-        const double2 o = pass == 1 ? make_double2(0.0, 0.0) : h[i];
-        h[i] = make_double2(o.x + d.x, o.y + d.y);
-        ss += d.x * d.x + d.y * d.y;
-    }
-    st->dloo = ss;
-    st->dnormw = sqrt(*norm2);
-    st->reorth = (2.0 * st->dnormw <= sqrt(ss) && pass < max_pass) ? 1 : 0;
-}
-
-// the rest of step j: h(j+1, j) = ||w||, the previous rotations, zrotg,
-// the rotation of the rhs column, bea = |g_{j+1}| / ||b||; the cycle stops
-// when bea <= tol, after m steps, or on a non-finite bea
-__global__ void k_gm_step(GmState *st, double2 *H, double *cs, double2 *sn, int j, int m, double tol) {
-    if (!st->active) return;
-    double2 *h = H + (size_t)j * (m + 1);
-    double2 *g = H + (size_t)m * (m + 1);
-    h[j + 1] = make_double2(st->dnormw, 0.0);
-    for (int i = 0; i < j; i++) zrot_dev(h[i], h[i + 1], cs[i], sn[i]);
-    {  // zrotg (classic reference algorithm)
-        const double2 a = h[j], b = h[j + 1];
-        double c;
-        double2 sv;
-        const double aa = cabs2(a);
-        if (aa == 0.0) {
-            c = 0.0;
-            sv = make_double2(1.0, 0.0);
-        } else {
-            const double scale = aa + cabs2(b);
-            const double a1 = cabs2(make_double2(a.x / scale, a.y / scale));
-            const double b1 = cabs2(make_double2(b.x / scale, b.y / scale));
-            const double nrm = scale * sqrt(a1 * a1 + b1 * b1);
-            const double2 alpha = make_double2(a.x / aa, a.y / aa);
-            c = aa / nrm;
-            const double2 t = cmul2(alpha, cconj2(b));
-            sv = make_double2(t.x / nrm, t.y / nrm);
-        }
-        cs[j] = c;
-        sn[j] = sv;
-    }
-    zrot_dev(g[j], g[j + 1], cs[j], sn[j]);
-    zrot_dev(h[j], h[j + 1], cs[j], sn[j]);
-    h[j + 1] = make_double2(0.0, 0.0);
-    const double bea = cabs2(g[j + 1]) / st->bn;
-    st->bea = bea;
-    st->iterations++;
-    st->jh = j + 1;
-    if (!isfinite(bea)) st->flags |= kGmNonFinite;
-    if (!(bea > tol && j + 1 < m)) st->active = 0;
-}
-
 // y = H(0:jh, 0:jh) \ g (upper triangular, SimplifiedZtrsv) into coef;
 // ncols = jh, or 0 when the solve ended before a cycle (zero rhs, exact
 // guess, non-finite)
 __global__ void k_gm_construct(GmState *st, const double2 *H, int m, double2 *coef) {
     const int jh = (st->flags & (kGmZero | kGmNonFinite)) || ((st->flags & kGmExact) && st->jh == 0) ? 0 : st->jh;
-    for (int i = 0; i < jh; i++) coef[i] = H[(size_t)m * (m + 1) + i];
+    __shared__ double2 y;
+    const int i = threadIdx.x;  // a thread per row
+    double2 c = i < jh ? H[(size_t)m * (m + 1) + i] : make_double2(0, 0);
+    const double2 d = i < jh ? H[(size_t)i * (m + 1) + i] : make_double2(1, 0);
+    double2 next = i < jh - 1 ? H[(size_t)(jh - 1) * (m + 1) + i] : make_double2(0, 0);
     for (int j = jh - 1; j >= 0; j--) {
-        double2 y = coef[j];
-        if (y.x != 0.0 || y.y != 0.0) {
-            y = cdiv<double>(y, H[(size_t)j * (m + 1) + j]);
-            coef[j] = y;
-            for (int i = j - 1; i >= 0; i--) {
-                const double2 t = cmul2(y, H[(size_t)j * (m + 1) + i]);
-                coef[i] = make_double2(coef[i].x - t.x, coef[i].y - t.y);
-            }
+        const double2 hij = next;
+        if (i < j - 1) next = H[(size_t)(j - 1) * (m + 1) + i];
+        if (i == j) {
+            if (c.x != 0.0 || c.y != 0.0) c = cdiv<double>(c, d);
+            y = c;
         }
+        __syncthreads();
+        const double2 v = y;
+        if (i < j && (v.x != 0.0 || v.y != 0.0)) {
+            const double2 t = cmul2(v, hij);
+            c = make_double2(c.x - t.x, c.y - t.y);
+        }
+        __syncthreads();
     }
-    st->ncols = jh;
+    if (i < jh) coef[i] = c;
+    if (i == 0) st->ncols = jh;
 }
 
 // true backward error ||b - A x|| / ||b||
@@ -804,7 +919,8 @@ __global__ void k_gm_count(const int *live, long long *count) {
 
 // an operator apply of the solve; in an enqueue-only solve it may be
 // speculative (its cycle already stopped): it runs all the same, but only a
-// live one is counted (on the device)
+// live one is counted (on the device; a step's own apply is counted by its
+// first dots)
 template <typename T>
 void Gmres<T>::apply_counted(const C<T> *x, C<T> *y, const int *live) {
     apply(x, y);
@@ -829,8 +945,8 @@ void Gmres<T>::reset_apply_counts() {
 
 template <typename T>
 void Gmres<T>::dc_norm(const C<T> *x, const int *live) {
-    VecOps<T>::norm2(x, n_, norm_dev_, reinterpret_cast<double *>(partials_), nblocks_, s_, live);
-    kernel_launches += 2;
+    VecOps<T>::norm2(x, n_, norm_dev_, scratch_, s_, live);
+    kernel_launches += 1;
 }
 
 template <typename T>
@@ -863,38 +979,35 @@ void Gmres<T>::dc_step(int j) {
     if (precond) {
         C<T> *zj = Z_ + (long)j * n_;
         precond(vj, zj);
-        apply_counted(zj, w_, live);
+        apply(zj, w_);
     } else {
-        apply_counted(vj, w_, live);
+        apply(vj, w_);
     }
     const int koff = sizeof(T) == sizeof(double) ? 0 : EGX_K_C64;
     for (int pass = 1; pass <= 3; pass++) {
         const int *p = pass == 1 ? live : more;
         int ev = timers ? timers->begin(EGX_K_GS_DOTS + koff, s_) : -1;
-        VecOps<T>::multi_dot(V_, j + 1, w_, n_, dots_, partials_, nblocks_, s_, p);
+        VecOps<T>::multi_dot(V_, j + 1, w_, n_, dots_, scratch_, s_, p,
+                             pass == 1 && enqueue_only ? napp_dev_ : nullptr);
         if (timers) timers->end(ev, s_);
         ev = timers ? timers->begin(EGX_K_GS_UPDATE + koff, s_) : -1;
-        VecOps<T>::update_norm(V_, j + 1, dots_, w_, n_, norm_dev_, reinterpret_cast<double *>(partials_), nblocks_,
-                               s_, p);
+        launch_update<T>(V_, j + 1, dots_, w_, n_, norm_dev_, scratch_, s_, p,
+                         GsControl{st_, Hd_, csd_, snd_, j, m_, pass, 3, tol_});
         if (timers) timers->end(ev, s_);
-        k_gm_ortho<<<1, 1, 0, s_>>>(st_, Hd_, dots_, norm_dev_, j, m_, pass, 3);
-        kernel_launches += 5;
+        kernel_launches += 2;
     }
-    if (j < m_ - 1) {
+    if (j < m_ - 1) {  // still active after the step
         VecOps<T>::divide_dev(w_, &st_->dnormw, V_ + (long)(j + 1) * n_, n_, s_, live);
         kernel_launches += 1;
     }
-    k_gm_step<<<1, 1, 0, s_>>>(st_, Hd_, csd_, snd_, j, m_, tol_);
-    kernel_launches += 1;
 }
 
 // ConstructCurrentSolution: result += (Z or V)[:, :jh] y
 template <typename T>
 void Gmres<T>::dc_construct(C<T> *result) {
-    k_gm_construct<<<1, 1, 0, s_>>>(st_, Hd_, m_, coef_);
-    VecOps<T>::gemv(precond ? Z_ : V_, m_, coef_, r0_, n_, s_, &st_->ncols);
-    VecOps<T>::add(r0_, result, n_, s_, &st_->ncols);
-    kernel_launches += 3;
+    k_gm_construct<<<1, 64, 0, s_>>>(st_, Hd_, m_, coef_);
+    VecOps<T>::gemv_add(precond ? Z_ : V_, m_, coef_, result, n_, s_, &st_->ncols);
+    kernel_launches += 2;
 }
 
 template <typename T>

@@ -12,19 +12,30 @@
 
 namespace egx {
 
+// Scratch of the vector sums: a row of partial sums per block (64 columns) and
+// the counter that finds a launch's last block, zero between launches.
+// Launches that share one must be ordered by a stream.
+struct GsScratch {
+    static constexpr int kMaxBlocks = 1024;
+    double2 *partials = nullptr;
+    unsigned *counter = nullptr;
+    int nblocks = 0;
+};
+
 // Vector kernels. `live` (device int, may be null): when it points at 0 the
 // launched kernel returns at once -- the predicated work of a Krylov cycle
 // that the host enqueued ahead of the device's decision to stop.
 template <typename T>
 struct VecOps {
-    // dots[k] = sum_r conj(V[r, k]) w[r] for k < ncols (V column-major, ld = n)
-    static void multi_dot(const C<T> *V, int ncols, const C<T> *w, long n, double2 *dots_dev, double2 *partials,
-                          int nblocks, cudaStream_t s, const int *live = nullptr);
+    // dots[k] = sum_r conj(V[r, k]) w[r] for k < ncols (V column-major, ld = n);
+    // *count (may be null) goes up by one
+    static void multi_dot(const C<T> *V, int ncols, const C<T> *w, long n, double2 *dots_dev, const GsScratch &g,
+                          cudaStream_t s, const int *live = nullptr, long long *count = nullptr);
     // w -= V[:, :ncols] * dots ; norm2_dev = ||w||^2
     static void update_norm(const C<T> *V, int ncols, const double2 *dots_dev, C<T> *w, long n, double *norm2_dev,
-                            double *partials, int nblocks, cudaStream_t s, const int *live = nullptr);
+                            const GsScratch &g, cudaStream_t s);
     // ||x||^2 into norm2_dev
-    static void norm2(const C<T> *x, long n, double *norm2_dev, double *partials, int nblocks, cudaStream_t s,
+    static void norm2(const C<T> *x, long n, double *norm2_dev, const GsScratch &g, cudaStream_t s,
                       const int *live = nullptr);
     // y = alpha * x (alpha real)
     static void scale(const C<T> *x, double alpha, C<T> *y, long n, cudaStream_t s);
@@ -34,12 +45,10 @@ struct VecOps {
     static void divide_dev(const C<T> *x, const double *d_dev, C<T> *y, long n, cudaStream_t s, const int *live);
     // y = a - b
     static void sub(const C<T> *a, const C<T> *b, C<T> *y, long n, cudaStream_t s, const int *live = nullptr);
-    // y += x
-    static void add(const C<T> *x, C<T> *y, long n, cudaStream_t s, const int *live = nullptr);
-    // out = V[:, :ncols] * coef (coef device); ncols_dev (device, may be null)
+    // y += V[:, :ncols] * coef (coef device); ncols_dev (device, may be null)
     // overrides ncols, and 0 columns launch nothing that writes
-    static void gemv(const C<T> *V, int ncols, const double2 *coef, C<T> *out, long n, cudaStream_t s,
-                     const int *ncols_dev = nullptr);
+    static void gemv_add(const C<T> *V, int ncols, const double2 *coef, C<T> *y, long n, cudaStream_t s,
+                         const int *ncols_dev = nullptr);
     static void copy(const C<T> *x, C<T> *y, long n, cudaStream_t s);
     static void zero(C<T> *x, long n, cudaStream_t s);
 };
@@ -57,7 +66,8 @@ struct GmresResult {
 
 // Device state of a device-controlled solve (Gmres::solve with
 // device_control): the scalars the reference's GmresSolver keeps in its
-// fields, updated by one-thread control kernels between the vector kernels.
+// fields, updated by control kernels and by the last blocks of the vector
+// kernels.
 struct GmState {
     double bn, beta, bea, dnormw, dloo, true_be;
     int active;      // the current cycle continues
@@ -89,8 +99,7 @@ class Gmres {
     long kernel_launches = 0;
     Timers *timers = nullptr;
     // Device control: the Arnoldi decisions (Gram-Schmidt passes, Givens
-    // rotations, stopping test, triangular solve) run in one-thread kernels
-    // on the device. With enqueue_only the whole solve (one cycle) is
+    // rotations, stopping test, triangular solve) run on the device. With enqueue_only the whole solve (one cycle) is
     // enqueued without any host wait -- the inner GMRES cycle of the
     // flexible preconditioner: steps after the device's stop are skipped by
     // their kernels, and the operator applies among them run speculatively
@@ -133,9 +142,9 @@ class Gmres {
     int max_restarts_;
     bool check_true_;
     cudaStream_t s_;
-    int nblocks_;
+    GsScratch scratch_;
     C<T> *V_ = nullptr, *Z_ = nullptr, *w_ = nullptr, *r0_ = nullptr, *xcur_ = nullptr;
-    double2 *dots_ = nullptr, *coef_ = nullptr, *partials_ = nullptr;
+    double2 *dots_ = nullptr, *coef_ = nullptr;
     double *norm_dev_ = nullptr;
     double *host_ = nullptr;  // pinned: dots + norm
     std::vector<std::complex<double>> H_;

@@ -56,7 +56,7 @@
 // 113-bit sums, nz = 1..48: 4e-17..2.9e-16, the FP64 kernel's 9e-17..3.4e-16.
 //
 // complex64 takes the packed layouts (the sub-block layout's own kernels are
-// faster at its layer counts: 254 us against 298 at 128x128x32). With four
+// faster at its layer counts: 110 us against 298 at 128x128x32). With four
 // digits the conversions of a tile (32 permutes and subtractions) cost as many
 // issue slots as its ten products take the tensor pipe, so two right-hand
 // sides share them: 180x120x35, two, 773 us against 978 one by one and
@@ -619,7 +619,8 @@ void launch_contract_dig(C<T> *buf, const void *dig, const OpDims &d, int *err, 
     const short *dexp = reinterpret_cast<const short *>(G + digit_bytes(GreenDims{d.nx, d.ny, d.nz}));
     // Registers for two blocks per SM where their shared memory fits too; a
     // third (48 registers a thread, or 56) spills: 637 us against 487 at
-    // 180x120x35, one right-hand side, 194 against 156 at 90x75x22, two.
+    // 180x120x35, one right-hand side, 194 against 156 at 90x75x22, two (142
+    // with the registers of five tiles' 320 threads).
     const int MT = dig_geom<T>(d.nz).MT;
     if constexpr (std::is_same<T, double>::value) {
         if (MT <= 6) launch<T, 1, 384, 2>(buf, G, dexp, d, err, s);
@@ -628,7 +629,8 @@ void launch_contract_dig(C<T> *buf, const void *dig, const OpDims &d, int *err, 
         if (MT <= 7) launch<T, 1, 448, 2>(buf, G, dexp, d, err, s);
         else launch<T, 1, 576, 2>(buf, G, dexp, d, err, s);
     } else {
-        if (MT <= 7) launch<T, 2, 448, 2>(buf, G, dexp, d, err, s);
+        if (MT <= 5) launch<T, 2, 320, 2>(buf, G, dexp, d, err, s);
+        else if (MT <= 7) launch<T, 2, 448, 2>(buf, G, dexp, d, err, s);
         else launch<T, 2, 576, 1>(buf, G, dexp, d, err, s);
     }
 }

@@ -28,18 +28,18 @@
 // Four kernels, one CTA per SM looping over stored points, the offsets of
 // each warp's A fragments held in registers (built once). The -A^T blocks
 // (z rows, x|y columns) take their sign on the B values.
-//  * k_contract_ws<NZ> (two right-hand sides, the stacked solve of both
-//    polarisations; built in): FP16 m16n8k16 with A fragments straight from
-//    the split entries, work split by role -- one warp per 16-row tile over
-//    all column tiles, two warps splitting the next point's right-hand
-//    sides, one producer lane (see the kernel).
+//  * k_contract_ws<NZ, NR> (built in, for the two right-hand sides of a
+//    stacked solve of both polarisations and for one): FP16 m16n8k16 with A
+//    fragments straight from the split entries, work split by role -- one
+//    warp per 16-row tile over all column tiles, two warps splitting the next
+//    point's right-hand sides, one producer lane (see the kernel).
 //  * k_contract_sh<NZ> (two; the tuner's variant 2): the same products with
 //    12 warps in lockstep, 3 row groups x 4 column groups, partial sums per
 //    row tile met in shared memory and added by the warps with the fewest
 //    column tiles.
 //  * k_contract_sb3<NZ> (two; variant 1) on the TF32 m16n8k8 path, the
 //    entries recombined to complex64 first, and k_contract_sb<NZ, 1> for one
-//    right-hand side.
+//    right-hand side (variant 1, and chi0 of the mixed form).
 //
 // Per stored point: one TMA bulk copy of the block (and, in the lockstep
 // and TF32 kernels, one per present right-hand-side segment) into one of
@@ -1019,12 +1019,16 @@ __global__ void __launch_bounds__(Sh<NZ>::THREADS, 1)
     }
 }
 
-// k_contract_ws<NZ>: the two-source FP16 split contraction with its work
-// split by role, so that the phases of one point overlap the products of
-// another instead of running in lockstep behind block barriers.
+// k_contract_ws<NZ, NR>: the FP16 split contraction of NR = 1 or 2 sources
+// with its work split by role, so that the phases of one point overlap the
+// products of another instead of running in lockstep behind block barriers.
 //  * MMA warps, one per row tile (MT of them): every k tile of their tile,
 //    12 products per k tile as in k_contract_sh, accumulators alternating
 //    by k tile; the output leaves from the accumulators (no partial sums).
+//    With one source the eight columns are the real and imaginary parts of
+//    its four points, Gr [Xr | Xi] and Gi [Xr | Xi]: six products per k
+//    tile, and lanes two apart exchange half of their sums, so that each
+//    finishes one row.
 //  * two split warps: load the right-hand sides of a point from global
 //    memory (the Green stage carries no right-hand sides), take one scale
 //    per column over all its rows, split into FP16 fragments in a double
@@ -1034,16 +1038,20 @@ __global__ void __launch_bounds__(Sh<NZ>::THREADS, 1)
 // Hand-offs are mbarriers; every wait is bounded, and a wait that gives up
 // records EGX_ERR_TIMEOUT and raises a block-wide abort flag that ends every
 // role's loop within one poll.
-template <int NZ>
+template <int NZ, int NR>
 struct Ws {
     static constexpr int R = 3 * NZ, MT = R / 16, KT = R / 16, BS = Sh<NZ>::BS;
     static constexpr int NSPLIT = 2, PRODUCER = MT + NSPLIT, THREADS = 32 * (MT + NSPLIT + 1);
     static constexpr int KPS = (KT + NSPLIT - 1) / NSPLIT;  // k tiles per split warp
     static constexpr uint32_t G_BYTES = BS * 8u;
-    static constexpr uint32_t BF_BYTES = KT * 2u * 32u * 16u;  // [KT][Xr, Xi][32 lanes] uint4
+    // [KT][Xr, Xi][32 lanes] uint4, or [KT][32 lanes] of [Xr | Xi]
+    static constexpr uint32_t BF_BYTES = KT * NR * 32u * 16u;
     static constexpr uint32_t OFF_BF = 2 * G_BYTES, OFF_INV = OFF_BF + 2 * BF_BYTES;
     static constexpr uint32_t OFF_MAX = OFF_INV + 2u * 8u * 4u;
     static constexpr uint32_t SMEM = OFF_MAX + 2u * NSPLIT * 8u * 4u;
+    // one source: two blocks per SM where their shared memory allows (its
+    // chains of products are half as long)
+    static constexpr int PER_SM = NR == 1 && 2 * (SMEM + 1280u) <= 228u * 1024u ? 2 : 1;
     static_assert(SMEM + 256 <= 227u * 1024u, "shared memory per block");
     static_assert(MT * KT * 2 * 32 * 4 <= G_BYTES, "offset scratch must fit in one stage");
     static_assert(G_BYTES % 128 == 0 && OFF_BF % 16 == 0, "stage alignment");
@@ -1078,11 +1086,11 @@ __device__ __forceinline__ bool ws_wait_warp(uint32_t bar, uint32_t parity, vola
     return __all_sync(0xffffffffu, ok);
 }
 
-template <int NZ>
-__global__ void __launch_bounds__(Ws<NZ>::THREADS, 1)
+template <int NZ, int NR>
+__global__ void __launch_bounds__(Ws<NZ, NR>::THREADS, Ws<NZ, NR>::PER_SM)
     k_contract_ws(float2 *buf, const float2 *__restrict__ G, const int nx, const int ny, const int B, const int rhs0,
                   int *err) {
-    using P = Ws<NZ>;
+    using P = Ws<NZ, NR>;
     constexpr int R = P::R, KT = P::KT;
     extern __shared__ __align__(128) unsigned char smem[];
     // [full, sempty, bfull, bempty, cmax] x 2: Green block landed, stage
@@ -1143,17 +1151,19 @@ __global__ void __launch_bounds__(Ws<NZ>::THREADS, 1)
                 break;
             const uint2 *Gq = reinterpret_cast<const uint2 *>(smem + s * P::G_BYTES);
             const uint4 *bfr = BFRAG + (size_t)s * (P::BF_BYTES / 16) + lane;
-            // T1 = Gr Xr, T2 = Gi Xi, T3 = Gr Xi, T4 = Gi Xr, even and odd k tiles
-            float acc[2][4][4];
+            // T1 = Gr Xr, T2 = Gi Xi, T3 = Gr Xi, T4 = Gi Xr, even and odd k
+            // tiles; one source: T1 = Gr [Xr | Xi], T2 = Gi [Xr | Xi]
+            constexpr int NT = 2 * NR;
+            float acc[2][NT][4];
 #pragma unroll
             for (int kt = 0; kt < KT; kt++) {
                 const uint32_t flip = (zrows && (16 * kt) / NZ < 2) ? 0x80008000u : 0u;
                 // B fragments [Xr, Xi][hi b0, hi b1, lo b0, lo b1]; the sign
                 // flips both FP16 halves (the split commutes with it)
-                uint32_t bf[2][4];
+                uint32_t bf[NR][4];
 #pragma unroll
-                for (int h = 0; h < 2; h++) {
-                    const uint4 f = bfr[(kt * 2 + h) * 32];
+                for (int h = 0; h < NR; h++) {
+                    const uint4 f = bfr[(kt * NR + h) * 32];
                     bf[h][0] = f.x ^ flip;
                     bf[h][1] = f.y ^ flip;
                     bf[h][2] = f.z ^ flip;
@@ -1173,22 +1183,18 @@ __global__ void __launch_bounds__(Ws<NZ>::THREADS, 1)
                     af[3][e] = __byte_perm(u.y, w.y, 0x7632);
                 }
                 float (*ac)[4] = acc[kt & 1];
+                // A part (high) and B operand of product j
+                auto ai = [](int j) { return NR == 1 ? 2 * j : ((j == 0 || j == 2) ? 0 : 2); };
+                auto bi = [](int j) { return NR == 1 ? 0 : ((j == 0 || j == 3) ? 0 : 1); };
 #pragma unroll
-                for (int j = 0; j < 4; j++) {
-                    const int ai = (j == 0 || j == 2) ? 0 : 2, bi = (j == 0 || j == 3) ? 0 : 1;
-                    if (kt < 2) mma_f16_zero(ac[j], af[ai], bf[bi][0], bf[bi][1]);
-                    else mma_f16(ac[j], af[ai], bf[bi][0], bf[bi][1]);
+                for (int j = 0; j < NT; j++) {
+                    if (kt < 2) mma_f16_zero(ac[j], af[ai(j)], bf[bi(j)][0], bf[bi(j)][1]);
+                    else mma_f16(ac[j], af[ai(j)], bf[bi(j)][0], bf[bi(j)][1]);
                 }
 #pragma unroll
-                for (int j = 0; j < 4; j++) {
-                    const int ai = (j == 0 || j == 2) ? 0 : 2, bi = (j == 0 || j == 3) ? 0 : 1;
-                    mma_f16(ac[j], af[ai], bf[bi][2], bf[bi][3]);
-                }
+                for (int j = 0; j < NT; j++) mma_f16(ac[j], af[ai(j)], bf[bi(j)][2], bf[bi(j)][3]);
 #pragma unroll
-                for (int j = 0; j < 4; j++) {
-                    const int ai = (j == 0 || j == 2) ? 1 : 3, bi = (j == 0 || j == 3) ? 0 : 1;
-                    mma_f16(ac[j], af[ai], bf[bi][0], bf[bi][1]);
-                }
+                for (int j = 0; j < NT; j++) mma_f16(ac[j], af[ai(j) + 1], bf[bi(j)][0], bf[bi(j)][1]);
             }
             // undo the scales of accumulator columns 2t and 2t + 1
             const float inv0 = INV[s * 8 + 2 * t], inv1 = INV[s * 8 + 2 * t + 1];
@@ -1197,8 +1203,36 @@ __global__ void __launch_bounds__(Ws<NZ>::THREADS, 1)
             const int a = (int)((unsigned)q / (unsigned)(ny + 1)), bq = q - a * (ny + 1);
             const int nkx = (a == 0 || a == nx) ? 1 : 2;
             const int nky = (bq == 0 || bq == ny) ? 1 : 2;
+            if constexpr (NR == 1) {
+                // lanes t < 2 hold columns of Xr, the others those of Xi of
+                // the same points: the first finish row g, the others row g + 8
+                const bool im = t >= 2;
 #pragma unroll
-            for (int c = 0; c < 4; c++) {
+                for (int c = 0; c < 2; c++) {
+                    float A[2], D[2];  // Gr x, Gi x of rows g, g + 8
+#pragma unroll
+                    for (int h = 0; h < 2; h++) {
+                        A[h] = acc[0][0][c + 2 * h] + acc[1][0][c + 2 * h];
+                        D[h] = acc[0][1][c + 2 * h] + acc[1][1][c + 2 * h];
+                    }
+                    const float oA = __shfl_xor_sync(0xffffffffu, im ? A[0] : A[1], 2);
+                    const float oD = __shfl_xor_sync(0xffffffffu, im ? D[0] : D[1], 2);
+                    const int row = 16 * mt + g + (im ? 8 : 0), v = 2 * (t & 1) + c;
+                    const int mx = v >> 1, my = v & 1;
+                    if (mx < nkx && my < nky) {
+                        const float f = c ? inv1 : inv0;
+                        float2 val = im ? make_float2((oA - D[1]) * f, (A[1] + oD) * f)
+                                        : make_float2((A[0] - oD) * f, (oA + D[0]) * f);
+                        const int comp = row / NZ;
+                        if ((comp == 0 && mx) || (comp == 1 && my)) val = make_float2(-val.x, -val.y);
+                        const long pt = (long)(mx ? 2 * nx - a : a) * n1 + (my ? 2 * ny - bq : bq);
+                        buf[pt * B + (long)rhs0 * R + row] = val;
+                    }
+                }
+                continue;
+            }
+#pragma unroll
+            for (int c = 0; c < 4 && NR == 2; c++) {
                 // rows g (c < 2) and g + 8 of the tile, column 2t + (c & 1):
                 // mirror point col & 3, source col >> 2
                 const int row = 16 * mt + g + 8 * (c >> 1);
@@ -1207,7 +1241,7 @@ __global__ void __launch_bounds__(Ws<NZ>::THREADS, 1)
                 if (mx < nkx && my < nky) {
                     const float f = (c & 1) ? inv1 : inv0;
                     const float t1 = acc[0][0][c] + acc[1][0][c], t2 = acc[0][1][c] + acc[1][1][c];
-                    const float t3 = acc[0][2][c] + acc[1][2][c], t4 = acc[0][3][c] + acc[1][3][c];
+                    const float t3 = acc[0][NT - 2][c] + acc[1][NT - 2][c], t4 = acc[0][NT - 1][c] + acc[1][NT - 1][c];
                     float2 val = make_float2((t1 - t2) * f, (t3 + t4) * f);
                     const int comp = row / NZ;
                     if ((comp == 0 && mx) || (comp == 1 && my)) val = make_float2(-val.x, -val.y);
@@ -1219,7 +1253,7 @@ __global__ void __launch_bounds__(Ws<NZ>::THREADS, 1)
     } else if (warp < P::PRODUCER) {
         // ---- split warp hh: k tiles hh, hh + NSPLIT, ... of every column
         const int hh = warp - P::MT;
-        const int bv = g & 3, brs = g >> 2, bmx = bv >> 1, bmy = bv & 1;
+        const int bv = g & 3, brs = NR == 1 ? 0 : g >> 2, bmx = bv >> 1, bmy = bv & 1;
         for (int it = 0, q = blockIdx.x; q < Q; q += gridDim.x, it++) {
             const int s = it & 1;
             const uint32_t par = (it >> 1) & 1;
@@ -1227,7 +1261,8 @@ __global__ void __launch_bounds__(Ws<NZ>::THREADS, 1)
             const int nkx = (a == 0 || a == nx) ? 1 : 2;
             const int nky = (bq == 0 || bq == ny) ? 1 : 2;
             const bool bpresent = bmx < nkx && bmy < nky;
-            // this lane's column: mirror point bv, source brs; rows
+            // this lane's column: mirror point bv, source brs (one source: the
+            // real part for g < 4, the imaginary one for the others); rows
             // 16 kt + 2t, +1 and 16 kt + 2t + 8, +9 with the D_p sign of
             // their component (loads issued before the buffer wait)
             float4 xv[P::KPS][2];
@@ -1282,6 +1317,16 @@ __global__ void __launch_bounds__(Ws<NZ>::THREADS, 1)
                 if (kt >= KT) continue;
                 // [Xr, Xi] x [hi b0, hi b1, lo b0, lo b1]
                 uint4 fr, fi;
+                if constexpr (NR == 1) {
+                    const bool im = g >= 4;
+#pragma unroll
+                    for (int h = 0; h < 2; h++) {
+                        const float u = im ? xv[i][h].y : xv[i][h].x, w = im ? xv[i][h].w : xv[i][h].z;
+                        split_h2(u * scB, w * scB, h ? fr.y : fr.x, h ? fr.w : fr.z);
+                    }
+                    bfw[kt * 32] = fr;
+                    continue;
+                }
                 split_h2(xv[i][0].x * scB, xv[i][0].z * scB, fr.x, fr.z);
                 split_h2(xv[i][1].x * scB, xv[i][1].z * scB, fr.y, fr.w);
                 split_h2(xv[i][0].y * scB, xv[i][0].w * scB, fi.x, fi.z);
@@ -1322,14 +1367,14 @@ void launch_sh(float2 *buf, const float2 *G, const OpDims &d, int rhs0, int *err
     EGX_CUDA(cudaGetLastError());
 }
 
-template <int NZ>
+template <int NZ, int NR>
 void launch_ws(float2 *buf, const float2 *G, const OpDims &d, int rhs0, int *err, cudaStream_t s, int nsm) {
-    using P = Ws<NZ>;
-    raise_smem_limit((const void *)k_contract_ws<NZ>, P::SMEM);
+    using P = Ws<NZ, NR>;
+    raise_smem_limit((const void *)k_contract_ws<NZ, NR>, P::SMEM);
     const long Q = (long)(d.nx + 1) * (d.ny + 1);
     EGX_CHECK(Q < (1L << 31), EGX_ERR_INVALID, "sub-block contraction: (nx + 1)(ny + 1) must be below 2^31");
-    const unsigned grid = (unsigned)std::min<long>(Q, nsm);
-    k_contract_ws<NZ><<<grid, P::THREADS, P::SMEM, s>>>(buf, G, d.nx, d.ny, d.B, rhs0, err);
+    const unsigned grid = (unsigned)std::min<long>(Q, (long)nsm * P::PER_SM);
+    k_contract_ws<NZ, NR><<<grid, P::THREADS, P::SMEM, s>>>(buf, G, d.nx, d.ny, d.B, rhs0, err);
     EGX_CUDA(cudaGetLastError());
 }
 
@@ -1354,11 +1399,13 @@ void launch_sb(float2 *buf, const float2 *G, const OpDims &d, int rhs0, int *err
 }
 
 template <int NZ>
-void launch_nz(float2 *buf, const float2 *G, const OpDims &d, int *err, cudaStream_t s, int nsm, long *launches) {
+void launch_nz(float2 *buf, const float2 *G, const OpDims &d, int *err, cudaStream_t s, int nsm, bool one_tf32,
+               long *launches) {
     // contract_variant: 1 k_contract_sb3 (TF32 split), 2 k_contract_sh
     // (FP16 split, all warps in lockstep), 0 the built-in choice:
     // k_contract_ws (FP16 split by role: 1.110 against 1.293 ms per
-    // two-source launch at 256x256x48)
+    // two-source launch at 256x256x48; one source at 128x128x32 110 us,
+    // 0.9 of the copy bandwidth, against 254 of k_contract_sb)
     const int v = d.contract_variant;
     for (int r0 = 0; r0 < d.nrhs;) {
         if (d.nrhs - r0 >= 2) {
@@ -1367,10 +1414,13 @@ void launch_nz(float2 *buf, const float2 *G, const OpDims &d, int *err, cudaStre
             else if (v == 2)
                 launch_sh<NZ>(buf, G, d, r0, err, s, nsm);
             else
-                launch_ws<NZ>(buf, G, d, r0, err, s, nsm);
+                launch_ws<NZ, 2>(buf, G, d, r0, err, s, nsm);
             r0 += 2;
         } else {
-            launch_sb<NZ, 1>(buf, G, d, r0, err, s, nsm);
+            if (v == 1 || one_tf32)
+                launch_sb<NZ, 1>(buf, G, d, r0, err, s, nsm);
+            else
+                launch_ws<NZ, 1>(buf, G, d, r0, err, s, nsm);
             r0 += 1;
         }
         if (launches) ++*launches;
@@ -1405,13 +1455,14 @@ void green_to_c64(const double2 *g64, float2 *g32, const GreenDims &gd, cudaStre
     if (launches) ++*launches;
 }
 
-void launch_contract_sb(float2 *buf, const float2 *G, const OpDims &d, int *err, cudaStream_t s, long *launches) {
+void launch_contract_sb(float2 *buf, const float2 *G, const OpDims &d, int *err, cudaStream_t s, bool one_tf32,
+                        long *launches) {
     static int nsm = 0;
     if (!nsm) EGX_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, 0));
     switch (d.nz) {
-        case 16: launch_nz<16>(buf, G, d, err, s, nsm, launches); break;
-        case 32: launch_nz<32>(buf, G, d, err, s, nsm, launches); break;
-        case 48: launch_nz<48>(buf, G, d, err, s, nsm, launches); break;
+        case 16: launch_nz<16>(buf, G, d, err, s, nsm, one_tf32, launches); break;
+        case 32: launch_nz<32>(buf, G, d, err, s, nsm, one_tf32, launches); break;
+        case 48: launch_nz<48>(buf, G, d, err, s, nsm, one_tf32, launches); break;
         default: throw Error(EGX_ERR_INVALID, "sub-block contraction needs nz in {16, 32, 48}");
     }
 }

@@ -543,7 +543,7 @@ void operator_apply(const OpDims &d, const OperatorData<T> &op, const C<T> *G, c
             // the complex64 copy is in the sub-block layout for these nz
             EGX_CHECK(err, EGX_ERR_INVALID, "complex64 contraction needs the device error flag");
             long extra = 0;
-            launch_contract_sb(reinterpret_cast<float2 *>(buf), reinterpret_cast<const float2 *>(G), d, err, s,
+            launch_contract_sb(reinterpret_cast<float2 *>(buf), reinterpret_cast<const float2 *>(G), d, err, s, !gen,
                                &extra);
             if (launches) *launches += extra - 1;
         } else if (std::is_same<T, double>::value && op.dig && err) {

@@ -16,7 +16,9 @@
 //              ScalarMathUtils.cs:243-263);
 //   k_hankel   the 431-tap digital filter and the post normalisation
 //              (HankelCoefficients.cs:103-118, ScalarMathUtils.cs:189-207);
-//   k_segments linear pieces per radius interval (ScalarSegments.cs:86-128);
+//   linear pieces per radius interval (ScalarSegments.cs:86-128): in FP64 as
+//              coefficients of the values at the radii, k_by_radius, in the
+//              mixed form as such, k_segments;
 //   k_cells    per (cell, block entry): signed sum of face integrals, written
 //              with the parity mirroring into the 2Nx x 2Ny grid
 //              (GreenTensorCalculator.cs:460-552, GreenTensorFftPopulator.cs:221-273);
@@ -370,11 +372,24 @@ __global__ void k_hankel(const double2 *__restrict__ U, int nu, int ntrans, long
     I[((long)u * ntrans + tr) * nrad + p.x] = dmk(sx / den, sy / den);
 }
 
-// IA/IB[u][seg][trans]; with IA32/IB32 also as float pairs {re h, re l,
-// im h, im l} for the double-FP32 face sums
+// IT[u][rad][trans] = I[u][trans][rad]: the FP64 face sums read a radius of
+// 32 transceivers at a time
+__global__ void __launch_bounds__(256) k_by_radius(const double2 *__restrict__ I, int ntrans, int nrad,
+                                                   double2 *__restrict__ IT) {
+    __shared__ double2 tile[32][33];
+    const int g0 = blockIdx.x * 32, t0 = blockIdx.y * 32, lane = threadIdx.x & 31;
+    const long u = (long)blockIdx.z * ntrans * nrad;
+    for (int k = threadIdx.x >> 5; k < 32; k += 8)
+        if (t0 + k < ntrans && g0 + lane < nrad) tile[k][lane] = I[u + (long)(t0 + k) * nrad + g0 + lane];
+    __syncthreads();
+    for (int k = threadIdx.x >> 5; k < 32; k += 8)
+        if (g0 + k < nrad && t0 + lane < ntrans) IT[u + (long)(g0 + k) * ntrans + t0 + lane] = tile[lane][k];
+}
+
+// the linear pieces of the radius intervals, IA/IB[u][seg][trans], as float
+// pairs {re h, re l, im h, im l} for the double-FP32 face sums
 __global__ void k_segments(const double2 *__restrict__ I, int nu, int ntrans, int nrad, const double *__restrict__ radii,
-                           double2 *__restrict__ IA, double2 *__restrict__ IB, float4 *__restrict__ IA32,
-                           float4 *__restrict__ IB32) {
+                           float4 *__restrict__ IA32, float4 *__restrict__ IB32) {
     long idx = (long)blockIdx.x * blockDim.x + threadIdx.x;
     const int nseg = nrad - 1;
     if (idx >= (long)nu * nseg * ntrans) return;
@@ -388,17 +403,13 @@ __global__ void k_segments(const double2 *__restrict__ I, int nu, int ntrans, in
     double2 a = dmk((v[sg + 1].x - v[sg].x) / div, (v[sg + 1].y - v[sg].y) / div);
     double2 bb = dsub(v[sg], dmul(a, dmk(sr, 0)));
     long o = ((long)u * nseg + sg) * ntrans + tr;
-    IA[o] = a;
-    IB[o] = bb;
-    if (IA32) {
-        float4 fa, fb;
-        ds_split(a.x, fa.x, fa.y);
-        ds_split(a.y, fa.z, fa.w);
-        ds_split(bb.x, fb.x, fb.y);
-        ds_split(bb.y, fb.z, fb.w);
-        IA32[o] = fa;
-        IB32[o] = fb;
-    }
+    float4 fa, fb;
+    ds_split(a.x, fa.x, fa.y);
+    ds_split(a.y, fa.z, fa.w);
+    ds_split(bb.x, fb.x, fb.y);
+    ds_split(bb.y, fb.z, fb.w);
+    IA32[o] = fa;
+    IB32[o] = fb;
 }
 
 struct Term {
@@ -407,46 +418,149 @@ struct Term {
     double wa, wb;
 };
 
-template <typename O> __device__ __forceinline__ O cell_out(double2 v);
-template <> __device__ __forceinline__ double2 cell_out<double2>(double2 v) { return v; }
+// The same sums by radius: a piece between radii r0, r1 is linear in its two
+// values, wa a + wb b = c0 v0 + c1 v1, and a cell's coefficients of one value
+// are added up (once per mesh, make_nodes). Two FP64 FMAs per value and entry instead of four
+// per piece: the FP64 pipes bound the sums (128x128x32, the six components
+// 2.06 ms against 4.18; the 15 of an E and an H level 1.78 against 3.16).
+struct Node {
+    long slot;  // source nrad + radius
+    double w;
+};
+
+// wa, wb of every term -> c0, c1
+__global__ void k_term_values(Term *terms, long n, const double *__restrict__ radii) {
+    const long e = (long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= n) return;
+    const Term t = terms[e];
+    const double r0 = radii[t.seg], c1 = (t.wa - t.wb * r0) / (radii[t.seg + 1] - r0);
+    terms[e].wa = t.wb - c1;
+    terms[e].wb = c1;
+}
+
+// A cell's terms by value, a warp per cell: a lane adds up the coefficients of
+// one value of the cell's range of radii, in the order of the terms. A face's
+// terms are a run of consecutive pieces, so a value's terms of a run are at
+// known places; the runs are found first. (Next to the source a cell has
+// hundreds of terms in them.) A cell has two faces in each direction, each in
+// at most two parts: eight runs. First the counts (WRITE false: ptr[cell +
+// 1]), then, with the rows' starts in ptr, the nodes.
+constexpr int kRuns = 8;
+template <bool WRITE>
+__global__ void k_term_nodes(const int *__restrict__ rowptr, const Term *__restrict__ terms, int ncell, int nsrc,
+                             int nrad, int *ptr, Node *__restrict__ nodes) {
+    const int cell = (int)(((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+    if (cell >= ncell) return;
+    const int e0 = rowptr[cell], e1 = rowptr[cell + 1];
+    int lo = nrad, hi = -1;
+    for (int e = e0 + lane; e < e1; e += 32) {
+        lo = min(lo, terms[e].seg);
+        hi = max(hi, terms[e].seg);
+    }
+    lo = __reduce_min_sync(0xffffffffu, lo);
+    hi = __reduce_max_sync(0xffffffffu, hi);
+    const int range = e1 > e0 ? hi - lo + 2 : 0;
+    __shared__ int run[8][kRuns + 1];
+    int *start = run[threadIdx.x >> 5], runs = 0;
+    for (int b = e0; b < e1; b += 32) {
+        const int e = b + lane;
+        const bool first =
+            e < e1 && (e == e0 || terms[e].src != terms[e - 1].src || terms[e].seg != terms[e - 1].seg + 1);
+        const unsigned m = __ballot_sync(0xffffffffu, first);
+        const int at = runs + __popc(m & ((1u << lane) - 1));
+        if (first && at < kRuns) start[at] = e;
+        runs += __popc(m);
+    }
+    runs = min(runs, kRuns);
+    if (lane == 0) start[runs] = e1;
+    __syncwarp();
+    int out = WRITE ? ptr[cell] : 0;
+    for (int i0 = 0; i0 < nsrc * range; i0 += 32) {
+        const int i = i0 + lane, src = i / range, node = lo + i - src * range;
+        double w = 0;
+        bool used = false;
+        for (int r = 0; r < runs; r++) {
+            const int es = start[r], len = start[r + 1] - es;
+            const int k = node - terms[es].seg;
+            if (terms[es].src != src || k < 0 || k > len) continue;
+            if (k >= 1) w += terms[es + k - 1].wb;
+            if (k < len) w += terms[es + k].wa;
+            used = true;
+        }
+        const unsigned m = __ballot_sync(0xffffffffu, used);
+        if (WRITE && used) nodes[out + __popc(m & ((1u << lane) - 1))] = Node{(long)src * nrad + node, w};
+        out += __popc(m);
+    }
+    if (!WRITE && lane == 0) ptr[cell + 1] = out;
+}
+
+// ptr[1..n] of counts -> their running sums, ptr[0] = 0 (one block)
+__global__ void __launch_bounds__(1024) k_running_sum(int *ptr, int n) {
+    __shared__ int warps[32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int base = 0;
+    for (int i0 = 0; i0 < n; i0 += 1024) {
+        const int i = i0 + threadIdx.x;
+        int v = i < n ? ptr[i + 1] : 0;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int u = __shfl_up_sync(0xffffffffu, v, o);
+            if (lane >= o) v += u;
+        }
+        if (lane == 31) warps[warp] = v;
+        __syncthreads();
+        int before = 0, all = 0;
+        for (int k = 0; k < 32; k++) {
+            if (k < warp) before += warps[k];
+            all += warps[k];
+        }
+        if (i < n) ptr[i + 1] = base + before + v;
+        base += all;
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) ptr[0] = 0;
+}
+
+// w . values at stride ntrans
+__device__ __forceinline__ double2 node_sum(const Node *__restrict__ nodes, int e0, int e1,
+                                            const double2 *__restrict__ IT, int ntrans) {
+    double2 acc = dmk(0, 0);
+#pragma unroll 4
+    for (int e = e0; e < e1; e++) {
+        const Node nd = nodes[e];
+        const double2 v = IT[nd.slot * ntrans];
+        acc.x = fma(nd.w, v.x, acc.x);
+        acc.y = fma(nd.w, v.y, acc.y);
+    }
+    return acc;
+}
 
 // Real-space value of each quadrant cell for block entries [t0, t0+tc),
 // written with the parity mirroring into buf[2nx][2ny][tc] (or only the
-// quadrant when compact), as complex128 or rounded to complex64.
-template <typename O>
-__global__ void k_cells(const int *__restrict__ rowptr, const Term *__restrict__ terms, const double2 *__restrict__ IA,
-                        const double2 *__restrict__ IB, int ntrans, int nseg, int nx, int ny, int t0, int tc, int xs,
-                        int ys, int compact, O *__restrict__ buf) {
+// quadrant when compact).
+__global__ void k_cells(const int *__restrict__ rowptr, const Node *__restrict__ nodes, const double2 *__restrict__ IT,
+                        int ntrans, int nx, int ny, int t0, int tc, int xs, int ys, int compact,
+                        double2 *__restrict__ buf) {
     const int cell = blockIdx.x;
     const int i = cell / ny, j = cell - (cell / ny) * ny;
     const int t = blockIdx.y * blockDim.x + threadIdx.x;
     if (t >= tc) return;
-    double2 acc = dmk(0, 0);
-    for (int e = rowptr[cell]; e < rowptr[cell + 1]; e++) {
-        const Term tm = terms[e];
-        long o = ((long)tm.src * nseg + tm.seg) * ntrans + t0 + t;
-        double2 a = IA[o], b = IB[o];
-        acc.x = fma(tm.wa, a.x, acc.x);
-        acc.y = fma(tm.wa, a.y, acc.y);
-        acc.x = fma(tm.wb, b.x, acc.x);
-        acc.y = fma(tm.wb, b.y, acc.y);
-    }
+    const double2 acc = node_sum(nodes, rowptr[cell], rowptr[cell + 1], IT + t0 + t, ntrans);
     if (compact) {
         // quadrant buffer [nx+1][ny+1][tc]: the mirror images are made by
         // the FFT's loads (fft_lines_sym)
-        buf[((long)i * (ny + 1) + j) * tc + t] = cell_out<O>(acc);
+        buf[((long)i * (ny + 1) + j) * tc + t] = acc;
         return;
     }
     const int n0 = 2 * nx, n1 = 2 * ny;
-    buf[((long)i * n1 + j) * tc + t] = cell_out<O>(acc);
+    buf[((long)i * n1 + j) * tc + t] = acc;
     if (i >= 1 && j >= 1) {
-        buf[((long)(n0 - i) * n1 + j) * tc + t] = cell_out<O>(dscal((double)xs, acc));
-        buf[((long)i * n1 + (n1 - j)) * tc + t] = cell_out<O>(dscal((double)ys, acc));
-        buf[((long)(n0 - i) * n1 + (n1 - j)) * tc + t] = cell_out<O>(dscal((double)(xs * ys), acc));
+        buf[((long)(n0 - i) * n1 + j) * tc + t] = dscal((double)xs, acc);
+        buf[((long)i * n1 + (n1 - j)) * tc + t] = dscal((double)ys, acc);
+        buf[((long)(n0 - i) * n1 + (n1 - j)) * tc + t] = dscal((double)(xs * ys), acc);
     } else if (i >= 1) {
-        buf[((long)(n0 - i) * n1) * tc + t] = cell_out<O>(dscal((double)xs, acc));
+        buf[((long)(n0 - i) * n1) * tc + t] = dscal((double)xs, acc);
     } else if (j >= 1) {
-        buf[((long)(n1 - j)) * tc + t] = cell_out<O>(dscal((double)ys, acc));
+        buf[((long)(n1 - j)) * tc + t] = dscal((double)ys, acc);
     }
 }
 
@@ -912,22 +1026,12 @@ __global__ void k_zero_rho(double2 *__restrict__ I, int nu, int ntrans, int nrad
 
 // Level tensor value of every cell of the full 2nx x 2ny offset grid for
 // transmitter layers [0, nt): buf[cell][nt] (cells without terms stay 0).
-template <typename O>
-__global__ void k_cells_level(const int *__restrict__ rowptr, const Term *__restrict__ terms,
-                              const double2 *__restrict__ IA, const double2 *__restrict__ IB, int ntrans, int nseg,
-                              int ncell, O *__restrict__ buf) {
+__global__ void k_cells_level(const int *__restrict__ rowptr, const Node *__restrict__ nodes,
+                              const double2 *__restrict__ IT, int ntrans, int ncell, double2 *__restrict__ buf) {
     const long idx = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= (long)ncell * ntrans) return;
     const int cell = (int)(idx / ntrans), t = (int)(idx - (long)cell * ntrans);
-    double2 acc = dmk(0, 0);
-    for (int e = rowptr[cell]; e < rowptr[cell + 1]; e++) {
-        const Term tm = terms[e];
-        const long o = ((long)tm.src * nseg + tm.seg) * ntrans + t;
-        const double2 a = IA[o], b = IB[o];
-        acc.x = fma(tm.wa, a.x, fma(tm.wb, b.x, acc.x));
-        acc.y = fma(tm.wa, a.y, fma(tm.wb, b.y, acc.y));
-    }
-    buf[idx] = cell_out<O>(acc);
+    buf[idx] = node_sum(nodes, rowptr[cell], rowptr[cell + 1], IT + t, ntrans);
 }
 
 // k_cells_level for the mixed form: Dot2 on float pairs, rounded to complex64
@@ -1151,6 +1255,30 @@ static void load_hankel_taps() {
     loaded.insert(dev);
 }
 
+// A component's term lists by value (see Node): uploaded to scratch, merged on
+// the device.
+void make_nodes(GreenWorkspace &w, GreenWorkspace::CellLists &cl, const std::vector<int> &rowptr,
+                const std::vector<Term> &terms, const double *radii_dev, int nrad, int nsrc, cudaStream_t s,
+                long *launches) {
+    const int ncell = (int)rowptr.size() - 1;
+    const long n = (long)terms.size();
+    const int *row = dev_upload(w.d_trow, rowptr, s);
+    Term *t = dev_upload(w.d_terms, terms, s);
+    cl.rowptr.ensure(rowptr.size() * sizeof(int));
+    int *ptr = cl.rowptr.as<int>();
+    const unsigned warps = (unsigned)(((long)ncell * 32 + 255) / 256);
+    k_term_values<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(t, n, radii_dev);
+    k_term_nodes<false><<<warps, 256, 0, s>>>(row, t, ncell, nsrc, nrad, ptr, nullptr);
+    k_running_sum<<<1, 1024, 0, s>>>(ptr, ncell);
+    int total = 0;
+    EGX_CUDA(cudaMemcpyAsync(&total, ptr + ncell, sizeof(int), cudaMemcpyDeviceToHost, s));
+    EGX_CUDA(cudaStreamSynchronize(s));
+    cl.terms.ensure(std::max(1, total) * sizeof(Node));
+    k_term_nodes<true><<<warps, 256, 0, s>>>(row, t, ncell, nsrc, nrad, ptr, cl.terms.as<Node>());
+    EGX_CUDA(cudaGetLastError());
+    if (launches) *launches += 4;
+}
+
 // The plan's items side by side: all lambdas and radii in one list each, so
 // that every stage is one launch over all of them.
 struct PlanLists {
@@ -1297,13 +1425,13 @@ void build_green(const GreenModel &m, int n_hankels, cudaStream_t s, DevBuf &qua
     GreenWorkspace local_ws;
     GreenWorkspace &w = ws ? *ws : local_ws;
     DevBuf &d_lay = w.d_lay, &d_trans = w.d_trans, &d_U = w.d_U, &d_I = w.d_I,
-           &d_flags = w.d_flags, &d_neg = w.d_neg, &d_radii = w.d_radii, &d_IA = w.d_IA, &d_IB = w.d_IB,
-           &d_buf = w.d_buf;
+           &d_flags = w.d_flags, &d_neg = w.d_neg, &d_radii = w.d_radii, &d_buf = w.d_buf;
     {
         std::vector<double> key = {(double)m.nx, (double)m.ny, m.dx, m.dy};
         key.insert(key.end(), radii.begin(), radii.end());
         if (key != w.key) {
-            for (bool &c : w.cached) c = false;
+            for (auto &form : w.cells)
+                for (auto &c : form) c.cached = false;
             w.key = key;
         }
     }
@@ -1355,21 +1483,20 @@ void build_green(const GreenModel &m, int n_hankels, cudaStream_t s, DevBuf &qua
         if (tm) tm->end(ev, s);
         if (launches) *launches += 2;
         const int nseg = nrad - 1;
-        d_IA.ensure((size_t)nu * nseg * ntrans * sizeof(double2));
-        d_IB.ensure((size_t)nu * nseg * ntrans * sizeof(double2));
         // the mixed form's face sums run in double-FP32 on float pairs
         const bool face_ds = lateral_fft32 && fft_lines_sym_ok<float>(p0, 0) && fft_lines_sym_ok<float>(p1, 0);
         if (face_ds) {
             w.d_IA32.ensure((size_t)nu * nseg * ntrans * sizeof(float4));
             w.d_IB32.ensure((size_t)nu * nseg * ntrans * sizeof(float4));
+            const long n = (long)nu * nseg * ntrans;
+            k_segments<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(d_I.as<double2>(), nu, ntrans, nrad, radii_dev,
+                                                                   w.d_IA32.as<float4>(), w.d_IB32.as<float4>());
+        } else {
+            w.d_IT.ensure((size_t)nu * nrad * ntrans * sizeof(double2));
+            k_by_radius<<<dim3((nrad + 31) / 32, (ntrans + 31) / 32, nu), 256, 0, s>>>(d_I.as<double2>(), ntrans, nrad,
+                                                                                       w.d_IT.as<double2>());
         }
-        {
-            long n = (long)nu * nseg * ntrans;
-            k_segments<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(
-                d_I.as<double2>(), nu, ntrans, nrad, radii_dev, d_IA.as<double2>(), d_IB.as<double2>(),
-                face_ds ? w.d_IA32.as<float4>() : nullptr, face_ds ? w.d_IB32.as<float4>() : nullptr);
-            if (launches) *launches += 1;
-        }
+        if (launches) *launches += 1;
         EGX_CUDA(cudaGetLastError());
         EGX_CUDA(cudaStreamSynchronize(s));
         if (stats) stats->ms_scalars += ms_since(t_half);
@@ -1401,34 +1528,37 @@ void build_green(const GreenModel &m, int n_hankels, cudaStream_t s, DevBuf &qua
         for (int ci = 0; ci < ncomp; ci++) {
             const int c = comps[ci];
             auto t_int = std::chrono::steady_clock::now();
-            if (!w.cached[c]) {
+            GreenWorkspace::CellLists &cl = w.cells[face_ds ? 1 : 0][c];
+            if (!cl.cached) {
                 // the term lists depend on the lateral mesh and radii only:
                 // made once and reused for every frequency of the model
                 std::vector<int> rowptr;
                 std::vector<Term> terms;
                 cell_terms(m, radii, c, slot, rowptr, terms);
-                dev_upload(w.rowptr[c], rowptr, s);
-                dev_upload(w.terms[c], terms, s);
+                if (face_ds) {
+                    dev_upload(cl.terms, terms, s);
+                    dev_upload(cl.rowptr, rowptr, s);
+                } else {
+                    make_nodes(w, cl, rowptr, terms, radii_dev, nrad, nu, s, launches);
+                }
                 EGX_CUDA(cudaStreamSynchronize(s));
-                w.nterms[c] = (long)terms.size();
-                w.cached[c] = true;
+                cl.nterms = (long)terms.size();
+                cl.cached = true;
             }
-            if (stats) stats->face_terms += w.nterms[c];
-            const int *drow = w.rowptr[c].as<int>();
-            const Term *dterm = w.terms[c].as<Term>();
+            if (stats) stats->face_terms += cl.nterms;
+            const int *drow = cl.rowptr.as<int>();
             for (int t0 = 0; t0 < blk; t0 += tc) {
                 const int tcc = std::min(tc, blk - t0);
                 if (!compact) EGX_CUDA(cudaMemsetAsync(d_buf.p, 0, (size_t)cells4 * tcc * sizeof(double2), s));
                 dim3 grid(m.nx * m.ny, (tcc + 127) / 128);
                 int ev = tm ? tm->begin(EGX_K_GREEN_CELLS, s) : -1;
                 if (fft32)
-                    k_cells_ds<<<grid, 128, 0, s>>>(drow, dterm, w.d_IA32.as<float4>(), w.d_IB32.as<float4>(),
+                    k_cells_ds<<<grid, 128, 0, s>>>(drow, cl.terms.as<Term>(), w.d_IA32.as<float4>(), w.d_IB32.as<float4>(),
                                                     ntrans, nseg, m.nx, m.ny, t0, tcc, px[c], py[c], 1,
                                                     w.d_buf32.as<float2>());
                 else
-                    k_cells<double2><<<grid, 128, 0, s>>>(drow, dterm, d_IA.as<double2>(), d_IB.as<double2>(), ntrans,
-                                                          nseg, m.nx, m.ny, t0, tcc, px[c], py[c], compact ? 1 : 0,
-                                                          d_buf.as<double2>());
+                    k_cells<<<grid, 128, 0, s>>>(drow, cl.terms.as<Node>(), w.d_IT.as<double2>(), ntrans, m.nx, m.ny, t0,
+                                                 tcc, px[c], py[c], compact ? 1 : 0, d_buf.as<double2>());
                 if (tm) tm->end(ev, s);
                 EGX_CUDA(cudaGetLastError());
                 ev = tm ? tm->begin(EGX_K_GREEN_FFT, s) : -1;
@@ -1591,35 +1721,39 @@ void build_level_green(const GreenModel &m, int n_hankels, double z, double shx,
         if (launches) *launches += 1;
     }
     const int nseg = nrad - 1;
-    w.d_IA.ensure((size_t)nu * nseg * ntrans * sizeof(double2));
-    w.d_IB.ensure((size_t)nu * nseg * ntrans * sizeof(double2));
     if (fft32) {
         w.d_IA32.ensure((size_t)nu * nseg * ntrans * sizeof(float4));
         w.d_IB32.ensure((size_t)nu * nseg * ntrans * sizeof(float4));
-    }
-    {
         const long n = (long)nu * nseg * ntrans;
-        k_segments<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(
-            w.d_I.as<double2>(), nu, ntrans, nrad, radii_dev, w.d_IA.as<double2>(), w.d_IB.as<double2>(),
-            fft32 ? w.d_IA32.as<float4>() : nullptr, fft32 ? w.d_IB32.as<float4>() : nullptr);
-        if (launches) *launches += 1;
+        k_segments<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(w.d_I.as<double2>(), nu, ntrans, nrad, radii_dev,
+                                                               w.d_IA32.as<float4>(), w.d_IB32.as<float4>());
+    } else {
+        w.d_IT.ensure((size_t)nu * nrad * ntrans * sizeof(double2));
+        k_by_radius<<<dim3((nrad + 31) / 32, (ntrans + 31) / 32, nu), 256, 0, s>>>(w.d_I.as<double2>(), ntrans, nrad,
+                                                                                   w.d_IT.as<double2>());
     }
+    if (launches) *launches += 1;
     EGX_CUDA(cudaGetLastError());
     // ---- face integration (term lists cached per geometry, shift and radii)
-    const int ncomp = level_components(kind);
+    const int ncomp = level_components(kind), form = fft32 ? 1 : 0;
     {
         std::vector<double> key = {(double)m.nx, (double)m.ny, m.dx, m.dy, shx, shy};
         key.insert(key.end(), radii.begin(), radii.end());
-        if (key != w.lkey[kind]) {
+        if (key != w.lkey[form][kind]) {
             std::vector<std::vector<int>> rp;
             std::vector<std::vector<Term>> tt;
             level_terms(m, radii, shx, shy, kind, ncomp, rp, tt);
             for (int c = 0; c < ncomp; c++) {
-                dev_upload(w.lrow[kind][c], rp[c], s);
-                dev_upload(w.lterm[kind][c], tt[c], s);
+                GreenWorkspace::CellLists &cl = w.lcells[form][kind][c];
+                if (fft32) {
+                    dev_upload(cl.terms, tt[c], s);
+                    dev_upload(cl.rowptr, rp[c], s);
+                } else {
+                    make_nodes(w, cl, rp[c], tt[c], radii_dev, nrad, nu, s, launches);
+                }
             }
             EGX_CUDA(cudaStreamSynchronize(s));
-            w.lkey[kind] = key;
+            w.lkey[form][kind] = key;
         }
     }
     const long ncell = 4L * m.nx * m.ny;
@@ -1633,14 +1767,14 @@ void build_level_green(const GreenModel &m, int n_hankels, double z, double shx,
     }
     for (int c = 0; c < ncomp; c++) {
         const long n = ncell * m.nz;
-        const int *rp = w.lrow[kind][c].as<int>();
-        const Term *tt = w.lterm[kind][c].as<Term>();
+        const GreenWorkspace::CellLists &cl = w.lcells[form][kind][c];
+        const int *rp = cl.rowptr.as<int>();
         if (fft32) {
             // face sums in double-FP32 rounded to complex64 as written, the
             // 2-D FFT in complex64, the tensor kept in complex64
             float2 *g32 = out.as<float2>() + (size_t)c * comp_elems;
             k_cells_level_ds<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(
-                rp, tt, w.d_IA32.as<float4>(), w.d_IB32.as<float4>(), ntrans, nseg, (int)ncell, g32);
+                rp, cl.terms.as<Term>(), w.d_IA32.as<float4>(), w.d_IB32.as<float4>(), ntrans, nseg, (int)ncell, g32);
             EGX_CUDA(cudaGetLastError());
             fft_lines<float>(g32, n0, (long)n1 * m.nz, m.nz, m.nz, n1, n1, p1, w.tw1_32.as<float2>(), -1, s, launches);
             fft_lines<float>(g32, n1, m.nz, (long)n1 * m.nz, m.nz, n0, n0, p0, w.tw0_32.as<float2>(), -1, s, launches);
@@ -1648,9 +1782,8 @@ void build_level_green(const GreenModel &m, int n_hankels, double z, double shx,
             continue;
         }
         double2 *g = out.as<double2>() + (size_t)c * comp_elems;
-        k_cells_level<double2><<<(unsigned)((n + 255) / 256), 256, 0, s>>>(rp, tt, w.d_IA.as<double2>(),
-                                                                           w.d_IB.as<double2>(), ntrans, nseg,
-                                                                           (int)ncell, g);
+        k_cells_level<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(rp, cl.terms.as<Node>(), w.d_IT.as<double2>(), ntrans,
+                                                                  (int)ncell, g);
         EGX_CUDA(cudaGetLastError());
         // PerformGreenTensorFft: the full 2-D transform of every layer column
         fft_lines<double>(g, n0, (long)n1 * m.nz, m.nz, m.nz, n1, n1, p1, w.tw1.as<double2>(), -1, s, launches);

@@ -31,19 +31,23 @@ struct GreenBuildStats {
 // scratch buffers, and per component the face-integration term lists (CSR),
 // which depend only on the lateral mesh and the radii -- not on frequency.
 struct GreenWorkspace {
-    DevBuf d_lam, d_lay, d_dec, d_diag, d_trans, d_U, d_I, d_rho, d_gidx, d_flags, d_neg, d_radii, d_IA, d_IB, d_buf,
-        tw0, tw1;
+    DevBuf d_lam, d_lay, d_dec, d_diag, d_trans, d_U, d_I, d_rho, d_gidx, d_flags, d_neg, d_radii, d_IT, d_buf, d_trow,
+        d_terms, tw0, tw1;
     DevBuf d_buf32, tw0_32, tw1_32;  // the complex64 lateral FFT of the mixed form
     int n64[2] = {0, 0}, n32[2] = {0, 0};  // lengths of the tables in tw0, tw1 and tw0_32, tw1_32
     DevBuf d_IA32, d_IB32;           // its face-sum coefficients as float pairs
+    // face sums of a component's cells (CSR): by radius (FP64), by piece (mixed form)
+    struct CellLists {
+        DevBuf rowptr, terms;
+        long nterms = 0;
+        bool cached = false;
+    };
     std::vector<double> key;  // nx, ny, dx, dy and the radii of the cached term lists
-    DevBuf rowptr[6], terms[6];
-    long nterms[6] = {};
-    bool cached[6] = {};
+    CellLists cells[2][6];
     // observation-level tensors (E: kind 0, H: kind 1): term lists per component,
     // keyed by the lateral mesh, the level's shift and the radii
-    std::vector<double> lkey[2];
-    DevBuf lrow[2][8], lterm[2][8];
+    std::vector<double> lkey[2][2];
+    CellLists lcells[2][2][8];
 };
 
 // Components of a level tensor: E (kind 0) xx yy zz xy xz yz zx zy, H (kind 1)

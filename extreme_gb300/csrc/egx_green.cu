@@ -82,12 +82,13 @@ struct LayerArgs {
     double2 zeta[kMaxLayers];
     double2 alpha_s[kMaxLayers];
     double2 beta_s[kMaxLayers];
+    double2 rzeta[kMaxLayers];  // 1 / zeta
     double thick[kMaxLayers];
     double tops[kMaxLayers + 1];
 };
 
 // Per lambda: eta, exp, P1, Q1, Ps, Qs over all layers. Arrays [6][L][nl]
-// (of the thirteen that k_chain_factors completes). A serial chain of FP64
+// (of the fourteen that k_chain_factors completes). A serial chain of FP64
 // divisions over the layers per lambda and mode (grid y): bound by latency, so
 // all plan items' lambdas go in one launch, in small blocks (5,350 lambdas,
 // 7 layers: 102 us; 20 launches of five blocks took 3,010).
@@ -161,15 +162,18 @@ struct Trans {
 // (1 + P_{k+1}) / (1 + P_k X_k), and F[k] = G[k] exp(z_{k+1} (eta_{k+1} -
 // eta_k)), so that a pair's chain A[t, b] = F[t] (... (F[b-1] H[b])) is a few
 // complex products; and the decay across a layer, Y[k] = exp(-(z_{k+1} - z_k)
-// eta_k). Arrays [mode][L][nl] after the six of k_layers: F at 6L nl, H at
-// 8L nl, G at 10L nl, then Y [L][nl] at 12L nl. A thread per layer and lambda.
-constexpr int kLayArrays = 13;
+// eta_k), and R[k] = 1 / eta_k (a complex quotient costs as much as the
+// products of a pair). Arrays [mode][L][nl] after the six of k_layers: F at
+// 6L nl, H at 8L nl, G at 10L nl, then Y [L][nl] at 12L nl and R at 13L nl. A
+// thread per layer and lambda.
+constexpr int kLayArrays = 14;
 __global__ void k_chain_factors(int nl, const LayerArgs a, double2 *__restrict__ lay) {
     const int m = blockIdx.x * blockDim.x + threadIdx.x;
     if (m >= nl) return;
     const int L = a.L, k = blockIdx.y;
     const long o = (long)k * nl + m;
     const double2 ek = lay[o], xk = lay[(long)L * nl + o];
+    lay[13L * L * nl + o] = drecip(ek);
     if (k + 1 < L) lay[12L * L * nl + o] = dexp(dscal(-(a.tops[k + 1] - a.tops[k]), ek));
     double2 ez = dmk(0, 0);
     if (k + 1 < L) ez = dexp(dscal(a.tops[k + 1], dsub(lay[o + nl], ek)));
@@ -208,9 +212,10 @@ __global__ void k_decays(int nl, const double2 *__restrict__ lay, const LayerArg
 // with the chain's exp(z_{k+1} (eta_{k+1} - eta_k)) multiplied out, every term
 // of a pair is a product of decays within the receiver's and transmitter's
 // layers and across the layers between, none of them above one. An
-// exponential is left for pairs in one background layer. FP64 pipes: 3.7 ms
-// for both tensor halves at 32 layers and 5,350 lambdas, against 8.0 with six
-// complex exponentials per pair and lambda.
+// exponential is left for pairs in one background layer, and no quotient. FP64
+// pipes: 2.3 ms for both tensor halves at 32 layers and 5,350 lambdas, against
+// 8.0 with six complex exponentials and up to four quotients per pair and
+// lambda.
 __global__ void k_kernels(const double *__restrict__ lam, int nl, const double2 *__restrict__ lay,
                           const double2 *__restrict__ dec, int nz, const LayerArgs a, const Trans *__restrict__ trans,
                           int ntrans, int which, double2 *__restrict__ U) {
@@ -293,8 +298,8 @@ __global__ void k_kernels(const double *__restrict__ lam, int nl, const double2 
         v = dadd(v, dmul(Q[(long)b * nl + m], Rr));
         return dadd(v, dscal(psisign, psi));
     };
-    const double2 annf = drecip(dmul(er, es));
-    const double2 zr2 = dscal(2.0, a.zeta[r]);
+    const double2 ir = lay[(13L * L + r) * nl + m], is = lay[(13L * L + s) * nl + m];
+    const double2 annf = dmul(ir, is), iz2 = dscal(0.5, a.rzeta[r]);
     long out = 0;
     double2 *Ub = U + (long)tr * nl + m;
     const long ustride = (long)ntrans * nl;
@@ -305,18 +310,18 @@ __global__ void k_kernels(const double *__restrict__ lam, int nl, const double2 
         Ub[ustride * out++] = u;
     }
     double2 anns = chain(1);
-    if (r > s) anns = dmul(ddiv(a.zeta[r], a.zeta[s]), anns);
+    if (r > s) anns = dmul(dmul(a.zeta[r], a.rzeta[s]), anns);
     if (which & 2) {
         double2 u = dmul(anns, special(Ps, Qs, 1, -1, psi1(Ps, Qs)));
-        Ub[ustride * out++] = ddiv(u, zr2);
+        Ub[ustride * out++] = dmul(u, iz2);
     }
     if (which & 4) {
-        double2 u = dmul(dmul(anns, drecip(es)), special(Ps, Qs, -1, 1, psi3(Ps, Qs)));
-        Ub[ustride * out++] = dmul(u, ddiv(dmk(l, 0), zr2));
+        double2 u = dmul(dmul(anns, is), special(Ps, Qs, -1, 1, psi3(Ps, Qs)));
+        Ub[ustride * out++] = dmul(u, dscal(l, iz2));
     }
     if (which & 8) {
-        double2 u = dmul(dmul(anns, drecip(er)), special(Ps, Qs, -1, -1, psi3(Ps, Qs)));
-        Ub[ustride * out++] = dmul(u, ddiv(dmk(-l, 0), zr2));
+        double2 u = dmul(dmul(anns, ir), special(Ps, Qs, -1, -1, psi3(Ps, Qs)));
+        Ub[ustride * out++] = dmul(u, dscal(-l, iz2));
     }
     if (which & 16) {
         double2 u;
@@ -337,7 +342,7 @@ __global__ void k_kernels(const double *__restrict__ lam, int nl, const double2 
         } else {
             u = dmul(dmul(anns, annf), special(Ps, Qs, 1, 1, psi1(Ps, Qs)));
         }
-        Ub[ustride * out++] = dmul(u, ddiv(dmk(l * l, 0), zr2));
+        Ub[ustride * out++] = dmul(u, dscal(l * l, iz2));
     }
 #undef E
 }
@@ -972,20 +977,21 @@ __global__ void k_kernels_vtp(const double *__restrict__ lam, int nl, const doub
         for (int k = b - 1; k >= t; k--) A = dmul(F[(long)k * nl + m], A);
         return A;
     };
-    const double2 er = E(r), es = E(s);
+    const double2 er = E(r);
     const double2 a1 = chain(0);
     double2 as = chain(1);
-    if (r > s) as = dmul(ddiv(a.zeta[r], a.zeta[s]), as);
+    if (r > s) as = dmul(dmul(a.zeta[r], a.rzeta[s]), as);
+    const double2 is = lay[(13L * L + s) * nl + m];
     const VtpTerms v1 = vtp_terms(Eta, P1, Q1, nl, m, a, T0, l);
     const VtpTerms vs = vtp_terms(Eta, Ps, Qs, nl, m, a, T0, l);
     auto pre = [&](const double2 *P, const double2 *Q, const VtpTerms &v, double psign) {
         return dadd(dmul(dscal(psign, P[(long)t * nl + m]), v.T), dmul(Q[(long)b * nl + m], v.R));
     };
     auto u1 = [&](const double2 *P, const double2 *Q, const VtpTerms &v, double2 A) {
-        return dmul(ddiv(A, es), dadd(pre(P, Q, v, 1), v.psi15));
+        return dmul(dmul(A, is), dadd(pre(P, Q, v, 1), v.psi15));
     };
     auto u3 = [&](const double2 *P, const double2 *Q, const VtpTerms &v, double2 A) {
-        return dmul(dmul(A, ddiv(er, es)), dadd(pre(P, Q, v, -1), v.psi34));
+        return dmul(dmul(A, dmul(er, is)), dadd(pre(P, Q, v, -1), v.psi34));
     };
     auto u4 = [&](const double2 *P, const double2 *Q, const VtpTerms &v, double2 A) {
         return dmul(A, dsub(pre(P, Q, v, -1), v.psi34));
@@ -993,13 +999,13 @@ __global__ void k_kernels_vtp(const double *__restrict__ lam, int nl, const doub
     double2 *Ub = U + (long)tr * nl + m;
     const long us = (long)ntrans * nl;
     if (kind == 0) {
-        const double2 zr2 = dscal(2.0, a.zeta[r]);
+        const double2 iz2 = dscal(0.5, a.rzeta[r]);
         Ub[0] = dmul(u1(P1, Q1, v1, a1), dmk(0.0, a.omega * kMu0 * 0.5));
-        Ub[us] = ddiv(dmul(dmul(as, er), dsub(pre(Ps, Qs, vs, 1), vs.psi15)), zr2);
-        Ub[2 * us] = dmul(u3(Ps, Qs, vs, as), ddiv(dmk(l, 0), zr2));
-        Ub[3 * us] = dmul(u4(Ps, Qs, vs, as), ddiv(dmk(-l, 0), zr2));
-        const double2 u5 = dmul(ddiv(as, es), dadd(pre(Ps, Qs, vs, 1), vs.psi5));
-        Ub[4 * us] = dmul(u5, ddiv(dmk(l * l, 0), zr2));
+        Ub[us] = dmul(dmul(dmul(as, er), dsub(pre(Ps, Qs, vs, 1), vs.psi15)), iz2);
+        Ub[2 * us] = dmul(u3(Ps, Qs, vs, as), dscal(l, iz2));
+        Ub[3 * us] = dmul(u4(Ps, Qs, vs, as), dscal(-l, iz2));
+        const double2 u5 = dmul(dmul(as, is), dadd(pre(Ps, Qs, vs, 1), vs.psi5));
+        Ub[4 * us] = dmul(u5, dscal(l * l, iz2));
     } else {
         Ub[0] = u3(P1, Q1, v1, a1);
         Ub[us] = u4(Ps, Qs, vs, as);
@@ -1337,6 +1343,8 @@ void build_green(const GreenModel &m, int n_hankels, cudaStream_t s, DevBuf &qua
     for (int k = 0; k < L; k++) {
         zb[k] = cd(m.bg_sigma[k], -m.omega * kEps0);
         la.zeta[k] = make_double2(zb[k].real(), zb[k].imag());
+        const cd rz = 1.0 / zb[k];
+        la.rzeta[k] = make_double2(rz.real(), rz.imag());
         la.thick[k] = m.bg_thick[k];
         la.tops[k] = tops[k];
     }
@@ -1623,6 +1631,8 @@ void build_level_green(const GreenModel &m, int n_hankels, double z, double shx,
     for (int k = 0; k < L; k++) {
         zb[k] = cd(m.bg_sigma[k], -m.omega * kEps0);
         la.zeta[k] = make_double2(zb[k].real(), zb[k].imag());
+        const cd rz = 1.0 / zb[k];
+        la.rzeta[k] = make_double2(rz.real(), rz.imag());
         la.thick[k] = m.bg_thick[k];
         la.tops[k] = tops[k];
     }

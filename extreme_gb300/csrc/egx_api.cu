@@ -24,14 +24,9 @@ int fail(egx_ctx *ctx, int code, const std::string &msg) {
 void set_device(egx_ctx *ctx) { EGX_CUDA(cudaSetDevice(ctx->device)); }
 
 void check_device_error(egx_ctx *ctx) {
-    int flag = 0;
-    EGX_CUDA(cudaMemcpyAsync(&flag, ctx->errflag.p, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
     EGX_CUDA(cudaStreamSynchronize(ctx->stream));
-    if (flag) {
-        EGX_CUDA(cudaMemsetAsync(ctx->errflag.p, 0, sizeof(int), ctx->stream));
-        EGX_CUDA(cudaStreamSynchronize(ctx->stream));
+    if (const int flag = ctx->errflag.take())
         throw Error(flag, "a device wait timed out (shared-memory pipeline did not complete)");
-    }
 }
 
 long nvec(const egx_ctx *ctx) { return (long)ctx->nx * ctx->ny * 3 * ctx->nz; }
@@ -392,7 +387,7 @@ void apply_dev(egx_ctx *ctx, const C<T> *x, C<T> *y, int nrhs, bool ds) {
     const C<T> *tw0 = dbl ? (const C<T> *)ctx->tw0_64.p : (const C<T> *)ctx->tw0_32.p;
     const C<T> *tw1 = dbl ? (const C<T> *)ctx->tw1_64.p : (const C<T> *)ctx->tw1_32.p;
     operator_apply<T>(d, op, G, x, y, buf.as<C<T>>(), tw0, tw1, ctx->p0, ctx->p1, ctx->stream, &ctx->launches,
-                      &ctx->timers, ctx->errflag.as<int>());
+                      &ctx->timers, ctx->errflag.device());
 }
 template void apply_dev<double>(egx_ctx *, const C<double> *, C<double> *, int, bool);
 template void apply_dev<float>(egx_ctx *, const C<float> *, C<float> *, int, bool);
@@ -562,8 +557,7 @@ int egx_create(int device, egx_ctx **out) {
         set_device(ctx);
         EGX_CUDA(cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking));
         ctx->own_stream = true;
-        ctx->errflag.ensure(sizeof(int));
-        EGX_CUDA(cudaMemset(ctx->errflag.p, 0, sizeof(int)));
+        ctx->errflag.create();
     } catch (const egx::Error &e) {
         delete ctx;
         return e.code;
@@ -1092,7 +1086,7 @@ int egx_wait_selftest(egx_ctx *ctx, double limit_ms) {
     EGX_GUARD(ctx, {
         EGX_CHECK(limit_ms >= 1 && limit_ms <= 2000, EGX_ERR_INVALID, "limit_ms must be in [1, 2000]");
         set_device(ctx);
-        k_wait_probe<<<1, 32, 0, ctx->stream>>>((uint64_t)(limit_ms * 1e6), ctx->errflag.as<int>());
+        k_wait_probe<<<1, 32, 0, ctx->stream>>>((uint64_t)(limit_ms * 1e6), ctx->errflag.device());
         ctx->launches++;
         EGX_CUDA(cudaGetLastError());
         EGX_CUDA(cudaStreamSynchronize(ctx->stream));

@@ -209,4 +209,28 @@ struct DevBuf {
     }
 };
 
+// An int that kernels write and the host reads, in pinned host memory: after a
+// synchronisation reading it is a load (a copy of a device int took 10 us of
+// every call that checks it).
+struct HostFlag {
+    int *p = nullptr;
+    HostFlag() {}
+    HostFlag(const HostFlag &) = delete;
+    HostFlag &operator=(const HostFlag &) = delete;
+    ~HostFlag() {
+        if (p) cudaFreeHost(p);
+    }
+    void create() {
+        EGX_CUDA(cudaHostAlloc((void **)&p, sizeof(int), cudaHostAllocMapped));
+        *p = 0;
+    }
+    int *device() const { return p; }  // one address space
+    int take() {
+        volatile int *f = p;
+        const int v = *f;
+        if (v) *f = 0;
+        return v;
+    }
+};
+
 }  // namespace egx

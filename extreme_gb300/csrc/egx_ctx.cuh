@@ -71,7 +71,7 @@ struct egx_ctx {
     long pc_nodes = 0, pc_replays = 0;
     egx::DevBuf nrm_part, nrm_counter, nrm_out, mix_r, mix_t, mix_r32, mix_d32;
     egx::DevBuf js, chi0;
-    egx::DevBuf errflag;  // device int: EGX_ERR_TIMEOUT from a bounded wait
+    egx::HostFlag errflag;  // EGX_ERR_TIMEOUT from a bounded wait
     egx::GreenBuildStats last_build;
     // observation level: transformed sources, 3-column results
     egx::DevBuf lvl_x, lvl_out, lvl_in, lvl_field;

@@ -230,7 +230,7 @@ __global__ void k_kernels(const double *__restrict__ lam, int nl, const double2 
 #define E(k) Eta[(long)(k) * nl + m]
     const int r = T0.r, s = T0.s, t = min(r, s), b = max(r, s);
     const double r1 = T0.r1, r2 = T0.r2;
-    const double2 er = E(r), es = E(s);
+    const double2 er = E(r);
     const double l = lam[m];
     // CalculateT / CalculateR and the C, D sums: signed sums of four
     // exponentials e^G (e^a - e^b)(e^c - e^d) over the receiver interval

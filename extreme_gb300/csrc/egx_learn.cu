@@ -560,7 +560,7 @@ int egx_net_create(egx_ctx *ctx, int nx, int ny, int nz, int width, int layers, 
         set_device(ctx);
         auto n = std::unique_ptr<egx_net>(new egx_net());
         n->nx = nx, n->ny = ny, n->nz = nz, n->W = width, n->L = layers;
-        n->err = ctx->errflag.as<int>();
+        n->err = ctx->errflag.device();
         n->fused = net_layer_fits(nz, width);
         n->cin = 7, n->cout = 6, n->ncell = (long)nx * ny;
         long off = 0;

@@ -17,7 +17,7 @@
 //
 // Measured at 8 samples of 128x128x32, W = 32, per layer (before: the strided
 // GEMM with element loads, k_gemm_bf16, and separate element-wise passes):
-//   lateral analysis   117 us (4.6 TB/s)                      before 391
+//   lateral analysis   98 us (5.5 TB/s)                       before 391
 //   layer sums         434 us forward (3.7 TB/s with the sums
 //                      before the activation kept), 340 us
 //                      backward (two blocks per SM; three spill:
@@ -88,7 +88,7 @@ __device__ __forceinline__ void a_fragments(uint4 *dst, int steps, int tid, int 
 // out[b][i][n] = sum_k bas[k][i] in[b][k][n], i < 16: the basis's columns
 // against K rows of N contiguous columns (rows ks apart). A warp per batch
 // item and 32 columns; the basis lies in shared memory as A fragments.
-__global__ void __launch_bounds__(256) k_analysis(const float *__restrict__ bas, const float *__restrict__ in, int K,
+__global__ void __launch_bounds__(256, 3) k_analysis(const float *__restrict__ bas, const float *__restrict__ in, int K,
                                                   long ks, long in_b, int N, long items, float *__restrict__ out) {
     extern __shared__ uint4 fr[];
     const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3, steps = (K + 15) / 16;
@@ -501,7 +501,7 @@ void net_analysis(const float *bas, int K, const float *in, long ks, long in_b, 
     const long items = batch * ((N + 31) / 32);
     const size_t bytes = (size_t)((K + 15) / 16) * 512;
     raise_smem_limit((const void *)k_analysis, bytes);
-    k_analysis<<<(unsigned)std::min<long>((items + 7) / 8, (long)sm_count() * 4), 256, bytes, s>>>(bas, in, K, ks, in_b,
+    k_analysis<<<(unsigned)std::min<long>((items + 7) / 8, (long)sm_count() * 3), 256, bytes, s>>>(bas, in, K, ks, in_b,
                                                                                                     N, items, out);
     EGX_CUDA(cudaGetLastError());
     if (launches) ++*launches;

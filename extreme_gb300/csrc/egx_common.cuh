@@ -209,6 +209,28 @@ struct DevBuf {
     }
 };
 
+// Kernels of a chain start while the one before runs out (programmatic
+// dependent launch): blocks become resident early and wait here for the
+// previous kernel's end and its writes, then let the next kernel do the same.
+// Every kernel launched with launch_after() calls after_previous() before it
+// touches memory and on every path, so the order of writes is that of plain
+// launches.
+__device__ __forceinline__ void after_previous() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+template <typename... P, typename... A>
+void launch_after(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args) {
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t c{};
+    c.gridDim = grid, c.blockDim = block, c.dynamicSmemBytes = smem, c.stream = s;
+    c.attrs = &at, c.numAttrs = 1;
+    EGX_CUDA(cudaLaunchKernelEx(&c, kernel, P(args)...));
+}
+
 // An int that kernels write and the host reads, in pinned host memory: after a
 // synchronisation reading it is a load (a copy of a device int took 10 us of
 // every call that checks it).

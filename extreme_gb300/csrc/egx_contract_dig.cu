@@ -401,6 +401,7 @@ __global__ void __launch_bounds__(MAXT, MINB)
             : "memory");
     };
     __syncthreads();
+    after_previous();
     if (tid == 0 && (int)blockIdx.x < Q) fetch(blockIdx.x);
 
     // this thread's right-hand-side entry: point xv, row xj
@@ -583,9 +584,8 @@ void launch(C<T> *buf, const unsigned char *G, const short *dexp, const OpDims &
     int per = 0;
     EGX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_contract_dig<T, NR, MAXT, MINB>, thr, m.bytes));
     const long Q = (long)(d.nx + 1) * (d.ny + 1);
-    k_contract_dig<T, NR, MAXT, MINB>
-        <<<(unsigned)std::min<long>(Q, (long)nsm * std::max(1, per)), thr, m.bytes, s>>>(buf, G, dexp, d, err);
-    EGX_CUDA(cudaGetLastError());
+    launch_after(k_contract_dig<T, NR, MAXT, MINB>, (unsigned)std::min<long>(Q, (long)nsm * std::max(1, per)), thr,
+                 m.bytes, s, buf, G, dexp, d, err);
 }
 
 }  // namespace

@@ -147,6 +147,7 @@ template <typename T>
 __global__ void k_multi_dot(const C<T> *__restrict__ V, int ncols, const C<T> *__restrict__ w, long n,
                             double2 *partials, double2 *__restrict__ out, unsigned *counter, const int *live,
                             long long *count) {
+    after_previous();
     if (live && !*live) return;
     if (count && blockIdx.x == 0 && threadIdx.x == 0) ++*count;
     constexpr int ROWS = DotRows<T>::value;
@@ -192,6 +193,7 @@ __global__ void k_multi_dot(const C<T> *__restrict__ V, int ncols, const C<T> *_
 __global__ void k_multi_dot_c2(const float4 *__restrict__ V, int ncols, const float4 *__restrict__ w, long n2,
                                double2 *partials, double2 *__restrict__ out, unsigned *counter, const int *live,
                                long long *count) {
+    after_previous();
     if (live && !*live) return;
     if (count && blockIdx.x == 0 && threadIdx.x == 0) ++*count;
     constexpr int ROWS = 4, kDotCols = 8;
@@ -376,6 +378,7 @@ struct GsControl {
 template <typename T>
 __global__ void k_update_norm(const C<T> *__restrict__ V, int ncols, const double2 *__restrict__ dots, C<T> *w, long n,
                               double *partials, double *out, unsigned *counter, const int *live, const GsControl gs) {
+    after_previous();
     if (live && !*live) {
         gs.skipped();
         return;
@@ -407,6 +410,7 @@ __global__ void k_update_norm(const C<T> *__restrict__ V, int ncols, const doubl
 __global__ void k_update_norm_c2(const float4 *__restrict__ V, int ncols, const double2 *__restrict__ dots, float4 *w,
                                  long n2, double *partials, double *out, unsigned *counter, const int *live,
                                  const GsControl gs) {
+    after_previous();
     if (live && !*live) {
         gs.skipped();
         return;
@@ -467,6 +471,7 @@ __global__ void k_divide(const C<T> *__restrict__ x, T d, C<T> *__restrict__ y, 
 template <typename T>
 __global__ void k_divide_dev(const C<T> *__restrict__ x, const double *__restrict__ d, C<T> *__restrict__ y, long n,
                              const int *live) {
+    after_previous();
     if (live && !*live) return;
     const T dd = (T)*d;
     for (long r = (long)blockIdx.x * blockDim.x + threadIdx.x; r < n; r += (long)gridDim.x * blockDim.x)
@@ -520,22 +525,22 @@ template <typename T>
 void VecOps<T>::multi_dot(const C<T> *V, int ncols, const C<T> *w, long n, double2 *dots_dev, const GsScratch &g,
                           cudaStream_t s, const int *live, long long *count) {
     if (sizeof(T) == sizeof(float) && n % 2 == 0 && aligned16(V) && aligned16(w))
-        k_multi_dot_c2<<<g.nblocks, kThreads, 0, s>>>(reinterpret_cast<const float4 *>(V), ncols,
-                                                      reinterpret_cast<const float4 *>(w), n / 2, g.partials, dots_dev,
-                                                      g.counter, live, count);
+        launch_after(k_multi_dot_c2, g.nblocks, kThreads, 0, s, reinterpret_cast<const float4 *>(V), ncols,
+                     reinterpret_cast<const float4 *>(w), n / 2, g.partials, dots_dev, g.counter, live, count);
     else
-        k_multi_dot<T><<<g.nblocks, kThreads, 0, s>>>(V, ncols, w, n, g.partials, dots_dev, g.counter, live, count);
+        launch_after(k_multi_dot<T>, g.nblocks, kThreads, 0, s, V, ncols, w, n, g.partials, dots_dev, g.counter, live,
+                     count);
 }
 template <typename T>
 static void launch_update(const C<T> *V, int ncols, const double2 *dots_dev, C<T> *w, long n, double *norm2_dev,
                           const GsScratch &g, cudaStream_t s, const int *live, const GsControl &gs) {
     double *part = reinterpret_cast<double *>(g.partials);
     if (sizeof(T) == sizeof(float) && n % 2 == 0 && aligned16(V) && aligned16(w))
-        k_update_norm_c2<<<g.nblocks, kThreads, 0, s>>>(reinterpret_cast<const float4 *>(V), ncols, dots_dev,
-                                                        reinterpret_cast<float4 *>(w), n / 2, part, norm2_dev,
-                                                        g.counter, live, gs);
+        launch_after(k_update_norm_c2, g.nblocks, kThreads, 0, s, reinterpret_cast<const float4 *>(V), ncols, dots_dev,
+                     reinterpret_cast<float4 *>(w), n / 2, part, norm2_dev, g.counter, live, gs);
     else
-        k_update_norm<T><<<g.nblocks, kThreads, 0, s>>>(V, ncols, dots_dev, w, n, part, norm2_dev, g.counter, live, gs);
+        launch_after(k_update_norm<T>, g.nblocks, kThreads, 0, s, V, ncols, dots_dev, w, n, part, norm2_dev, g.counter,
+                     live, gs);
 }
 template <typename T>
 void VecOps<T>::update_norm(const C<T> *V, int ncols, const double2 *dots_dev, C<T> *w, long n, double *norm2_dev,
@@ -556,7 +561,7 @@ void VecOps<T>::divide(const C<T> *x, double d, C<T> *y, long n, cudaStream_t s)
 }
 template <typename T>
 void VecOps<T>::divide_dev(const C<T> *x, const double *d, C<T> *y, long n, cudaStream_t s, const int *live) {
-    k_divide_dev<T><<<grid_for(n), kThreads, 0, s>>>(x, d, y, n, live);
+    launch_after(k_divide_dev<T>, grid_for(n), kThreads, 0, s, x, d, y, n, live);
 }
 template <typename T>
 void VecOps<T>::sub(const C<T> *a, const C<T> *b, C<T> *y, long n, cudaStream_t s, const int *live) {

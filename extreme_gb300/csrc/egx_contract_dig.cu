@@ -584,7 +584,7 @@ void launch(C<T> *buf, const unsigned char *G, const short *dexp, const OpDims &
     int per = 0;
     EGX_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_contract_dig<T, NR, MAXT, MINB>, thr, m.bytes));
     const long Q = (long)(d.nx + 1) * (d.ny + 1);
-    launch_after(k_contract_dig<T, NR, MAXT, MINB>, (unsigned)std::min<long>(Q, (long)nsm * std::max(1, per)), thr,
+    launch_after(buffer_bytes<T>(d), k_contract_dig<T, NR, MAXT, MINB>, (unsigned)std::min<long>(Q, (long)nsm * std::max(1, per)), thr,
                  m.bytes, s, buf, G, dexp, d, err);
 }
 

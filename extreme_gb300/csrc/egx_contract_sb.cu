@@ -1093,6 +1093,7 @@ __global__ void __launch_bounds__(Ws<NZ, NR>::THREADS, Ws<NZ, NR>::PER_SM)
     using P = Ws<NZ, NR>;
     constexpr int R = P::R, KT = P::KT;
     extern __shared__ __align__(128) unsigned char smem[];
+    after_previous();
     // [full, sempty, bfull, bempty, cmax] x 2: Green block landed, stage
     // read, fragments split, fragments read, split warps' column maxima
     __shared__ __align__(8) uint64_t bars[10];
@@ -1374,8 +1375,7 @@ void launch_ws(float2 *buf, const float2 *G, const OpDims &d, int rhs0, int *err
     const long Q = (long)(d.nx + 1) * (d.ny + 1);
     EGX_CHECK(Q < (1L << 31), EGX_ERR_INVALID, "sub-block contraction: (nx + 1)(ny + 1) must be below 2^31");
     const unsigned grid = (unsigned)std::min<long>(Q, (long)nsm * P::PER_SM);
-    k_contract_ws<NZ, NR><<<grid, P::THREADS, P::SMEM, s>>>(buf, G, d.nx, d.ny, d.B, rhs0, err);
-    EGX_CUDA(cudaGetLastError());
+    launch_after(buffer_bytes<float>(d), k_contract_ws<NZ, NR>, grid, P::THREADS, P::SMEM, s, buf, G, d.nx, d.ny, d.B, rhs0, err);
 }
 
 template <int NZ, bool BAL>

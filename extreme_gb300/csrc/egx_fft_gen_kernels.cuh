@@ -99,7 +99,7 @@ bool gen_fwd_y(const FftPlan &p, const C<T> *x, const OperatorData<T> &op, C<T> 
     auto run = [&](auto cls) {
         constexpr int K = decltype(cls)::value;
         raise_smem_limit((const void *)k_fwd_y_g<T, K>, l.smem);
-        launch_after(k_fwd_y_g<T, K>, gen_grid(d.B, l.lbt, d.nx), l.threads, l.smem, s, x, op, buf, d, p.gen, tw, l.lbt);
+        launch_after(buffer_bytes<T>(d), k_fwd_y_g<T, K>, gen_grid(d.B, l.lbt, d.nx), l.threads, l.smem, s, x, op, buf, d, p.gen, tw, l.lbt);
     };
     by_class(p.gen, run);
     return true;
@@ -113,7 +113,7 @@ bool gen_bwd_y(const FftPlan &p, const C<T> *buf, const C<T> *x, const OperatorD
     auto run = [&](auto cls) {
         constexpr int K = decltype(cls)::value;
         raise_smem_limit((const void *)k_bwd_y_g<T, K>, l.smem);
-        launch_after(k_bwd_y_g<T, K>, gen_grid(d.B, l.lbt, d.nx), l.threads, l.smem, s, buf, x, op, y, d, p.gen, tw, l.lbt);
+        launch_after(buffer_bytes<T>(d), k_bwd_y_g<T, K>, gen_grid(d.B, l.lbt, d.nx), l.threads, l.smem, s, buf, x, op, y, d, p.gen, tw, l.lbt);
     };
     by_class(p.gen, run);
     return true;
@@ -127,7 +127,7 @@ bool gen_lines(const FftPlan &p, C<T> *buf, int nlines, long lstride, long estri
     auto run = [&](auto cls) {
         constexpr int K = decltype(cls)::value;
         raise_smem_limit((const void *)k_lines_g<T, K>, l.smem);
-        launch_after(k_lines_g<T, K>, gen_grid(B, l.lbt, nlines), l.threads, l.smem, s, buf, lstride, estride, B, nload,
+        launch_after((size_t)nlines * p.n * B * sizeof(C<T>), k_lines_g<T, K>, gen_grid(B, l.lbt, nlines), l.threads, l.smem, s, buf, lstride, estride, B, nload,
                      nstore, p.gen, tw, l.lbt, sign);
     };
     by_class(p.gen, run);

@@ -525,10 +525,10 @@ template <typename T>
 void VecOps<T>::multi_dot(const C<T> *V, int ncols, const C<T> *w, long n, double2 *dots_dev, const GsScratch &g,
                           cudaStream_t s, const int *live, long long *count) {
     if (sizeof(T) == sizeof(float) && n % 2 == 0 && aligned16(V) && aligned16(w))
-        launch_after(k_multi_dot_c2, g.nblocks, kThreads, 0, s, reinterpret_cast<const float4 *>(V), ncols,
+        launch_after((size_t)n * ncols * sizeof(C<T>), k_multi_dot_c2, g.nblocks, kThreads, 0, s, reinterpret_cast<const float4 *>(V), ncols,
                      reinterpret_cast<const float4 *>(w), n / 2, g.partials, dots_dev, g.counter, live, count);
     else
-        launch_after(k_multi_dot<T>, g.nblocks, kThreads, 0, s, V, ncols, w, n, g.partials, dots_dev, g.counter, live,
+        launch_after((size_t)n * ncols * sizeof(C<T>), k_multi_dot<T>, g.nblocks, kThreads, 0, s, V, ncols, w, n, g.partials, dots_dev, g.counter, live,
                      count);
 }
 template <typename T>
@@ -536,10 +536,10 @@ static void launch_update(const C<T> *V, int ncols, const double2 *dots_dev, C<T
                           const GsScratch &g, cudaStream_t s, const int *live, const GsControl &gs) {
     double *part = reinterpret_cast<double *>(g.partials);
     if (sizeof(T) == sizeof(float) && n % 2 == 0 && aligned16(V) && aligned16(w))
-        launch_after(k_update_norm_c2, g.nblocks, kThreads, 0, s, reinterpret_cast<const float4 *>(V), ncols, dots_dev,
+        launch_after((size_t)n * ncols * sizeof(C<T>), k_update_norm_c2, g.nblocks, kThreads, 0, s, reinterpret_cast<const float4 *>(V), ncols, dots_dev,
                      reinterpret_cast<float4 *>(w), n / 2, part, norm2_dev, g.counter, live, gs);
     else
-        launch_after(k_update_norm<T>, g.nblocks, kThreads, 0, s, V, ncols, dots_dev, w, n, part, norm2_dev, g.counter,
+        launch_after((size_t)n * ncols * sizeof(C<T>), k_update_norm<T>, g.nblocks, kThreads, 0, s, V, ncols, dots_dev, w, n, part, norm2_dev, g.counter,
                      live, gs);
 }
 template <typename T>
@@ -561,7 +561,7 @@ void VecOps<T>::divide(const C<T> *x, double d, C<T> *y, long n, cudaStream_t s)
 }
 template <typename T>
 void VecOps<T>::divide_dev(const C<T> *x, const double *d, C<T> *y, long n, cudaStream_t s, const int *live) {
-    launch_after(k_divide_dev<T>, grid_for(n), kThreads, 0, s, x, d, y, n, live);
+    launch_after((size_t)n * sizeof(C<T>), k_divide_dev<T>, grid_for(n), kThreads, 0, s, x, d, y, n, live);
 }
 template <typename T>
 void VecOps<T>::sub(const C<T> *a, const C<T> *b, C<T> *y, long n, cudaStream_t s, const int *live) {

@@ -137,6 +137,7 @@ __global__ void __launch_bounds__(reg_threads<N, T, BT>(), reg_min_blocks<N, T, 
     k_fwd_y_r(const C<T> *__restrict__ x, const OperatorData<T> op, C<T> *__restrict__ buf, const OpDims d,
               const C<T> *__restrict__ tw) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
+    after_previous();
     const int i = blockIdx.y;
     const int b = blockIdx.x * BT + (int)(threadIdx.x % BT);
     const bool bok = b < d.B;
@@ -160,6 +161,7 @@ __global__ void __launch_bounds__(reg_threads<N, T, BT>())
     k_lines_r(C<T> *buf, long lstride, long estride, int B, int nload, int nstore, const C<T> *__restrict__ tw,
               int sign) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
+    after_previous();
     const int b = blockIdx.x * BT + (int)(threadIdx.x % BT);
     const bool bok = b < B;
     C<T> *line = buf + (long)blockIdx.y * lstride + b;
@@ -175,6 +177,7 @@ __global__ void __launch_bounds__(reg_threads<N, T, BT>(), reg_min_blocks<N, T, 
     k_bwd_y_r(const C<T> *__restrict__ buf, const C<T> *__restrict__ x, const OperatorData<T> op,
               C<T> *__restrict__ y, const OpDims d, const C<T> *__restrict__ tw) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
+    after_previous();
     const int i = blockIdx.y;
     const int b = blockIdx.x * BT + (int)(threadIdx.x % BT);
     const bool bok = b < d.B;
@@ -238,13 +241,13 @@ static void launch_reg(int which, cudaStream_t s, int nlines, const C<T> *x, con
     const dim3 grid((B + BT - 1) / BT, nlines);
     if (which == 0) {
         reg_attr<T, N, BT>((const void *)k_fwd_y_r<T, N, BT>);
-        k_fwd_y_r<T, N, BT><<<grid, thr, sm, s>>>(x, *op, buf, *d, tw);
+        launch_after(buffer_bytes<T>(*d), k_fwd_y_r<T, N, BT>, grid, thr, sm, s, x, *op, buf, *d, tw);
     } else if (which == 1) {
         reg_attr<T, N, BT>((const void *)k_lines_r<T, N, BT>);
-        k_lines_r<T, N, BT><<<grid, thr, sm, s>>>(buf, lstride, estride, B, nload, nstore, tw, sign);
+        launch_after((size_t)nlines * N * B * sizeof(C<T>), k_lines_r<T, N, BT>, grid, thr, sm, s, buf, lstride, estride, B, nload, nstore, tw, sign);
     } else {
         reg_attr<T, N, BT>((const void *)k_bwd_y_r<T, N, BT>);
-        k_bwd_y_r<T, N, BT><<<grid, thr, sm, s>>>(buf, x, *op, y, *d, tw);
+        launch_after(buffer_bytes<T>(*d), k_bwd_y_r<T, N, BT>, grid, thr, sm, s, buf, x, *op, y, *d, tw);
     }
 }
 

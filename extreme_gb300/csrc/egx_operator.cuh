@@ -38,6 +38,9 @@ struct OpDims {
     int contract_variant = 0;
 };
 
+// the spectral buffer
+template <typename T> size_t buffer_bytes(const OpDims &d) { return (size_t)4 * d.nx * d.ny * d.B * sizeof(C<T>); }
+
 template <typename T>
 struct OperatorData {
     const C<T> *r;    // [nx*ny*nz]

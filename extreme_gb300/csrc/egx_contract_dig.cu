@@ -1,7 +1,6 @@
 // Block contraction of the CIE operator (ConvolutionOperator.ApplyGreenTensorAlongZ,
 // ConvolutionOperator.cs:274-327) with error-free digit products on the FP16
-// tensor cores: complex128, and complex64 of the layer counts without the
-// sub-block layout.
+// tensor cores, complex128.
 //
 // GB300 issues two FP64 FMAs per clock and SM, so the block product in FP64
 // arithmetic is bound by them; its tensor cores multiply small FP16 integers
@@ -54,15 +53,6 @@
 // products alone need 0.29 ms (2,592 MMAs per point at 8 cycles per
 // sub-partition); the rest is the phases between them. 2-norm error against
 // 113-bit sums, nz = 1..48: 4e-17..2.9e-16, the FP64 kernel's 9e-17..3.4e-16.
-//
-// complex64 takes the packed layouts (the sub-block layout's own kernels are
-// faster at its layer counts: 110 us against 298 at 128x128x32). With four
-// digits the conversions of a tile (32 permutes and subtractions) cost as many
-// issue slots as its ten products take the tensor pipe, so two right-hand
-// sides share them: 180x120x35, two, 773 us against 978 one by one and
-// 1,640 us of the FP32 kernel (k_contract_c64); one, 487 us. 2-norm error
-// 2e-8..1e-7 where the FP32 kernel's is 4e-8..1.8e-7; 2e-7 against 1e-7 only
-// where a vector falls by 40 decades over the layers.
 #include <cuda_fp16.h>
 
 #include <algorithm>
@@ -617,24 +607,10 @@ template <typename T>
 void launch_contract_dig(C<T> *buf, const void *dig, const OpDims &d, int *err, cudaStream_t s) {
     const unsigned char *G = static_cast<const unsigned char *>(dig);
     const short *dexp = reinterpret_cast<const short *>(G + digit_bytes(GreenDims{d.nx, d.ny, d.nz}));
-    // Registers for two blocks per SM where their shared memory fits too; a
-    // third (48 registers a thread, or 56) spills: 637 us against 487 at
-    // 180x120x35, one right-hand side, 194 against 156 at 90x75x22, two (142
-    // with the registers of five tiles' 320 threads).
     const int MT = dig_geom<T>(d.nz).MT;
-    if constexpr (std::is_same<T, double>::value) {
-        if (MT <= 6) launch<T, 1, 384, 2>(buf, G, dexp, d, err, s);
-        else launch<T, 1, 576, 1>(buf, G, dexp, d, err, s);
-    } else if (d.nrhs == 1) {
-        if (MT <= 7) launch<T, 1, 448, 2>(buf, G, dexp, d, err, s);
-        else launch<T, 1, 576, 2>(buf, G, dexp, d, err, s);
-    } else {
-        if (MT <= 5) launch<T, 2, 320, 2>(buf, G, dexp, d, err, s);
-        else if (MT <= 7) launch<T, 2, 448, 2>(buf, G, dexp, d, err, s);
-        else launch<T, 2, 576, 1>(buf, G, dexp, d, err, s);
-    }
+    if (MT <= 6) launch<T, 1, 384, 2>(buf, G, dexp, d, err, s);
+    else launch<T, 1, 576, 1>(buf, G, dexp, d, err, s);
 }
 template void launch_contract_dig<double>(double2 *, const void *, const OpDims &, int *, cudaStream_t);
-template void launch_contract_dig<float>(float2 *, const void *, const OpDims &, int *, cudaStream_t);
 
 }  // namespace egx

@@ -551,8 +551,8 @@ void operator_apply(const OpDims &d, const OperatorData<T> &op, const C<T> *G, c
             if (launches) *launches += extra - 1;
         } else if (std::is_same<T, double>::value && op.dig && err) {
             launch_contract_dig<double>(reinterpret_cast<double2 *>(buf), op.dig, d, err, s);
-        } else if (std::is_same<T, float>::value && op.dig && err && gen && d.contract_variant == 0) {
-            launch_contract_dig<float>(reinterpret_cast<float2 *>(buf), op.dig, d, err, s);
+        } else if (std::is_same<T, float>::value && err && gen && d.contract_variant == 0 && contract_b3_fits(d.nz)) {
+            launch_contract_b3(reinterpret_cast<float2 *>(buf), reinterpret_cast<const float2 *>(G), d, err, s);
         } else if (std::is_same<T, float>::value && err && d.contract_variant == 0 && contract_mma_fits(d.nz, d.nrhs)) {
             launch_contract_mma(reinterpret_cast<float2 *>(buf), reinterpret_cast<const float2 *>(G), d, err, s);
         } else if (std::is_same<T, float>::value && err && d.contract_variant != 2 && contract_c64_fits(d.nz, d.nrhs)) {

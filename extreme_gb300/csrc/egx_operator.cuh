@@ -60,8 +60,8 @@ void operator_apply(const OpDims &d, const OperatorData<T> &op, const C<T> *G, c
 // vectors fit in 96 KiB
 bool contract_ds_fits(int nz, int nrhs);
 
-// contraction with error-free digit products on the tensor cores
-// (egx_contract_dig.cu): complex128, and complex64 of the packed layout. It
+// complex128 contraction with error-free digit products on the tensor cores
+// (egx_contract_dig.cu). It
 // reads a copy of the tensor in digits that digitise() makes once per tensor
 // (contract_dig_bytes() of it).
 bool contract_dig_fits(int nz);
@@ -69,6 +69,11 @@ size_t contract_dig_bytes(const GreenDims &gd);
 void digitise(const double2 *g64, void *out, const GreenDims &gd, cudaStream_t s, long *launches);
 template <typename T>
 void launch_contract_dig(C<T> *buf, const void *dig, const OpDims &d, int *err, cudaStream_t s);
+
+// complex64 contraction of the packed layout on the BF16 tensor cores
+// (egx_contract_b3.cu)
+bool contract_b3_fits(int nz);
+void launch_contract_b3(float2 *buf, const float2 *G, const OpDims &d, int *err, cudaStream_t s);
 
 // complex64 contraction with TMA-staged blocks (egx_contract.cu); `err`
 // receives EGX_ERR_TIMEOUT if a bounded wait expires.

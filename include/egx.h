@@ -135,7 +135,7 @@ int egx_graph_stats(egx_ctx *ctx, long *replays, long *nodes);
  * (complex64 Green tensor), times `reps` complex64 applies of nrhs vectors
  * for every kernel variant -- the FFT passes' column tile (0 built-in per
  * pass, 1 64-byte, 2 128-byte) x the contraction kernel: for the packed
- * Green layout 0 built-in order (digit products on the tensor cores), 1
+ * Green layout 0 built-in order (BF16 parts on the tensor cores), 1
  * TMA-staged CUDA-core, 2 generic; for the
  * sub-block layout of nz in {16, 32, 48} 0 built-in (FP16 split, warps by
  * role), 1 TF32 split, 2 FP16 split in lockstep -- keeps the fastest for the

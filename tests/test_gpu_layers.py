@@ -1,0 +1,60 @@
+"""GPU: the error of each layer of an apply by itself. A source in one layer,
+or one that falls by many decades over the layers, makes responses of very
+different size, and the small ones are to be as accurate as the large ones.
+
+Tolerance, of each layer's own 2-norm: complex64 inputs, the two transforms of
+12 and 10 points (16 stages) and results at 2^-24, doubled for the stages'
+constants: 2.2e-6.
+"""
+import numpy as np
+import pytest
+
+from extreme_gb300 import egx
+from extreme_gb300.model import OmegaModel, freq_to_omega, random_model
+from oracle import operator as op
+
+pytestmark = pytest.mark.gpu
+
+
+def _case(ctx, nz, f, seed):
+    m = random_model(6, 5, nz, seed=seed, n_boxes=0)
+    m.sigma = m.sigma * 10.0 ** np.random.default_rng(seed).uniform(-1, 1, m.sigma.shape)
+    om = OmegaModel.build(m, f)
+    g = ctx.green_build(m, freq_to_omega(f), 10)
+    G = g.download()
+    g.free()
+    return m, om, G
+
+
+def _sources(m, nz, rng, kind):
+    x = rng.standard_normal((m.nx, m.ny, 3, nz)) + 1j * rng.standard_normal((m.nx, m.ny, 3, nz))
+    if kind == "one layer":
+        w = np.zeros(nz)
+        w[nz // 4] = 1.0
+    else:  # down and up again by twelve decades
+        w = 10.0 ** (-12.0 * np.abs(np.sin(np.arange(nz) * 2.0)))
+    return (x * w).reshape(-1)
+
+
+def _layer_errors(y, want, m, nz):
+    d = (np.asarray(y, complex) - want).reshape(m.nx * m.ny * 3, nz)
+    return np.linalg.norm(d, axis=0) / np.linalg.norm(want.reshape(m.nx * m.ny * 3, nz), axis=0)
+
+
+@pytest.mark.parametrize("nz,f", [(9, 0.1), (22, 0.1), (24, 10.0), (35, 1.0), (47, 0.1)])
+@pytest.mark.parametrize("kind", ["one layer", "falling"])
+def test_every_layer_in_complex64(egx_ctx, nz, f, kind):
+    """The packed layouts, one and two right-hand sides."""
+    m, om, G = _case(egx_ctx, nz, f, nz)
+    g = egx_ctx.green_upload(G, m.nx, m.ny, nz, precision=egx.PREC_MIXED)
+    try:
+        egx_ctx.op_prepare(g, om.zeta, om.zeta0, m.layer_thickness, op.OP_A)
+        rng = np.random.default_rng(nz)
+        xs = [_sources(m, nz, rng, kind).astype(np.complex64), _sources(m, nz, rng, "falling").astype(np.complex64)]
+        for nrhs in (1, 2):
+            y = egx_ctx.op_apply_c64(np.concatenate(xs[:nrhs]), nrhs=nrhs).reshape(nrhs, -1)
+            for i in range(nrhs):
+                err = _layer_errors(y[i], op.apply(G, om, xs[i].astype(complex), op.OP_A), m, nz)
+                assert err.max() < 2.2e-6, (nrhs, i, err)
+    finally:
+        g.free()

@@ -77,24 +77,6 @@ void gather_quadrant(int nx, int ny, int nz, const double *const comps[6], std::
         }
 }
 
-// The digit copy of a tensor, where the digit contraction takes it: with the
-// tensor, but for mixed ones in the sub-block layout on their first complex128
-// apply (their inner applies do not read it). Without the memory for it the
-// contraction stays on the kernels that need none.
-void make_digits(egx_ctx *ctx, egx_green *g) {
-    if (g->dig.p || g->no_dig || !contract_dig_fits(g->nz)) return;
-    GreenDims gd{g->nx, g->ny, g->nz};
-    g->dig.swap(ctx->spare_dig);
-    try {
-        g->dig.ensure(contract_dig_bytes(gd));
-    } catch (const Error &) {
-        cudaGetLastError();
-        g->no_dig = true;
-        return;
-    }
-    digitise(g->g64.as<double2>(), g->dig.p, gd, ctx->stream, &ctx->launches);
-}
-
 // the context's scratch of vector sums (on its stream)
 GsScratch sum_scratch(egx_ctx *ctx, int nblocks) {
     if (!ctx->nrm_counter.p) {
@@ -191,8 +173,8 @@ GmresResult run_fgmres(egx_ctx *ctx, const C<T> *b, C<T> *x, int m_out, int m_in
             (*outer)->precond = [ctx, in, vb, tol, nrhs](const C<T> *src, C<T> *dst) {
                 C<T> *pin = ctx->pc_in.as<C<T>>(), *pout = ctx->pc_out.as<C<T>>();
                 char key[512];
-                snprintf(key, sizeof key, "%p/%p/%p/%p/%p/%p/%p/%p/%p/%p/%p/%p/%d/%d/%.17g/%zu/%d/%d", (void *)in, ctx->g,
-                         ctx->g->g32.p, ctx->g->g64.p, ctx->g->dig.p, ctx->r32.p, ctx->r64.p, ctx->buf32.p, ctx->buf64.p,
+                snprintf(key, sizeof key, "%p/%p/%p/%p/%p/%p/%p/%p/%p/%p/%p/%d/%d/%.17g/%zu/%d/%d", (void *)in, ctx->g,
+                         ctx->g->g32.p, ctx->g->g64.p, ctx->r32.p, ctx->r64.p, ctx->buf32.p, ctx->buf64.p,
                          ctx->tw0_32.p, (void *)pin, (void *)pout, ctx->type, nrhs, tol, vb, ctx->fft_tile,
                          ctx->contract_variant);
                 EGX_CUDA(cudaMemcpyAsync(pin, src, vb, cudaMemcpyDeviceToDevice, ctx->stream));
@@ -381,8 +363,6 @@ void apply_dev(egx_ctx *ctx, const C<T> *x, C<T> *y, int nrhs, bool ds) {
         op.bwd = (const C<T> *)ctx->bwd32.p;
     }
     op.type = ctx->type;
-    if (dbl) make_digits(ctx, ctx->g);
-    op.dig = ctx->g->dig.p;
     const C<T> *G = dbl ? (const C<T> *)ctx->g->g64.p : (const C<T> *)ctx->g->g32.p;
     const C<T> *tw0 = dbl ? (const C<T> *)ctx->tw0_64.p : (const C<T> *)ctx->tw0_32.p;
     const C<T> *tw1 = dbl ? (const C<T> *)ctx->tw1_64.p : (const C<T> *)ctx->tw1_32.p;
@@ -749,7 +729,6 @@ int egx_green_build(egx_ctx *ctx, const egx_model *model, double omega, int n_ha
         // the mixed form transforms the FP64 face integrals laterally in complex64
         build_green(gm, n_hankels, ctx->stream, g->g64, &st, &ctx->launches, &ctx->timers, &ctx->gws,
                     precision == EGX_PREC_MIXED);
-        if (precision != EGX_PREC_MIXED || !sb_layout(g->nz)) make_digits(ctx, g.get());
         if (precision == EGX_PREC_MIXED) {
             GreenDims gd{gm.nx, gm.ny, gm.nz};
             g->g32.swap(ctx->spare32);
@@ -778,7 +757,6 @@ int egx_green_upload(egx_ctx *ctx, int nx, int ny, int nz, const double *const c
         g->nz = nz;
         g->g64.ensure(q.size() * sizeof(cd));
         EGX_CUDA(cudaMemcpyAsync(g->g64.p, q.data(), q.size() * sizeof(cd), cudaMemcpyHostToDevice, ctx->stream));
-        if (precision != EGX_PREC_MIXED || !sb_layout(nz)) make_digits(ctx, g.get());
         if (precision == EGX_PREC_MIXED) {
             GreenDims gd{nx, ny, nz};
             g->g32.ensure(green_c64_entries(gd) * sizeof(float2));
@@ -854,7 +832,6 @@ int egx_green_free(egx_ctx *ctx, egx_green *g) {
     // follows, one frequency after another); egx_destroy releases it
     if (!ctx->spare64.p) ctx->spare64.swap(g->g64);
     if (!ctx->spare32.p) ctx->spare32.swap(g->g32);
-    if (!ctx->spare_dig.p) ctx->spare_dig.swap(g->dig);
     delete g;
     return EGX_OK;
 }

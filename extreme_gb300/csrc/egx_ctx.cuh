@@ -15,8 +15,6 @@ struct egx_green {
     int nx = 0, ny = 0, nz = 0;
     egx::DevBuf g64;  // quadrant, complex128
     egx::DevBuf g32;  // quadrant, complex64 (mixed precision)
-    egx::DevBuf dig;  // g64 in digits, for the complex128 contraction (where contract_dig_fits)
-    bool no_dig = false;  // no memory for them
     bool has32 = false;
 };
 
@@ -30,7 +28,7 @@ struct egx_ctx {
     // Green-tensor build workspace, and the storage of the last freed tensor
     // (reused by the next build of the same size; released by egx_destroy)
     egx::GreenWorkspace gws;
-    egx::DevBuf spare64, spare32, spare_dig;
+    egx::DevBuf spare64, spare32;
 
     // prepared operator
     egx_green *g = nullptr;

@@ -366,8 +366,8 @@ __global__ void k_contract(C<T> *buf, const C<T> *__restrict__ G, const OpDims d
 
 // ---------------------------------------------------------------------------
 // The complex128 contraction in double-FP32 arithmetic: the mixed form's
-// refinement residual where the digit products do not take it (nz > 48, or no
-// memory for the digit copy). GB300 runs complex128 FMAs at 1/64 of the FP32 rate,
+// refinement residual where the digit products do not take it (nz > 48). GB300
+// runs complex128 FMAs at 1/64 of the FP32 rate,
 // which makes the FP64 block product above compute-bound; here every
 // operand is a pair of floats hi + lo (47 significant bits) and every dot
 // product runs as Dot2 (Ogita, Rump and Oishi, "Accurate sum and dot
@@ -549,8 +549,8 @@ void operator_apply(const OpDims &d, const OperatorData<T> &op, const C<T> *G, c
             launch_contract_sb(reinterpret_cast<float2 *>(buf), reinterpret_cast<const float2 *>(G), d, err, s, !gen,
                                &extra);
             if (launches) *launches += extra - 1;
-        } else if (std::is_same<T, double>::value && op.dig && err) {
-            launch_contract_dig<double>(reinterpret_cast<double2 *>(buf), op.dig, d, err, s);
+        } else if (std::is_same<T, double>::value && err && contract_dig_fits(d.nz)) {
+            launch_contract_dig(reinterpret_cast<double2 *>(buf), reinterpret_cast<const double2 *>(G), d, err, s);
         } else if (std::is_same<T, float>::value && err && gen && d.contract_variant == 0 && contract_b3_fits(d.nz)) {
             launch_contract_b3(reinterpret_cast<float2 *>(buf), reinterpret_cast<const float2 *>(G), d, err, s);
         } else if (std::is_same<T, float>::value && err && d.contract_variant == 0 && contract_mma_fits(d.nz, d.nrhs)) {

@@ -47,7 +47,6 @@ struct OperatorData {
     const C<T> *fwd;  // [nz]
     const C<T> *bwd;  // [nz]
     int type;         // EGX_OP_A / EGX_OP_CHI0
-    const void *dig = nullptr;  // digit copy of the tensor (digitise)
 };
 
 // Launch the full apply y = K x (nrhs vectors) on `stream`.
@@ -61,14 +60,9 @@ void operator_apply(const OpDims &d, const OperatorData<T> &op, const C<T> *G, c
 bool contract_ds_fits(int nz, int nrhs);
 
 // complex128 contraction with error-free digit products on the tensor cores
-// (egx_contract_dig.cu). It
-// reads a copy of the tensor in digits that digitise() makes once per tensor
-// (contract_dig_bytes() of it).
+// (egx_contract_dig.cu)
 bool contract_dig_fits(int nz);
-size_t contract_dig_bytes(const GreenDims &gd);
-void digitise(const double2 *g64, void *out, const GreenDims &gd, cudaStream_t s, long *launches);
-template <typename T>
-void launch_contract_dig(C<T> *buf, const void *dig, const OpDims &d, int *err, cudaStream_t s);
+void launch_contract_dig(double2 *buf, const double2 *G, const OpDims &d, int *err, cudaStream_t s);
 
 // complex64 contraction of the packed layout on the BF16 tensor cores
 // (egx_contract_b3.cu)

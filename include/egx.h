@@ -183,11 +183,10 @@ int egx_op_apply(egx_ctx *ctx, const double *x, double *y, int nrhs, int where);
 int egx_op_apply_c64(egx_ctx *ctx, const float *x, float *y, int nrhs, int where);
 /* The apply the mixed form uses for its refinement residuals: a complex128
  * apply whose block contraction needs no complex128 FMA. For nz <= 48 it is
- * egx_op_apply's own (error-free digit products); beyond, or without the
- * memory for the digit copy, double-FP32 arithmetic (Dot2 on float pairs,
- * ~47 significant bits) for nz <= 53 and 4 nrhs 3 nz float4 of staged
- * vectors <= 96 KiB, else the complex128 contraction. Same arguments as
- * egx_op_apply. */
+ * egx_op_apply's own (error-free digit products); beyond, double-FP32
+ * arithmetic (Dot2 on float pairs, ~47 significant bits) for nz <= 53 and
+ * 4 nrhs 3 nz float4 of staged vectors <= 96 KiB, else the complex128
+ * contraction. Same arguments as egx_op_apply. */
 int egx_op_apply_ds(egx_ctx *ctx, const double *x, double *y, int nrhs, int where);
 
 /* ---- FFT (FftWrap plan_many_dft rank 2) -------------------------------- */

@@ -2,9 +2,10 @@
 or one that falls by many decades over the layers, makes responses of very
 different size, and the small ones are to be as accurate as the large ones.
 
-Tolerance, of each layer's own 2-norm: complex64 inputs, the two transforms of
-12 and 10 points (16 stages) and results at 2^-24, doubled for the stages'
-constants: 2.2e-6.
+Tolerances, of each layer's own 2-norm: complex128 both sides round at 2^-53,
+at most 300 terms and 40 operations of the transforms, (300 + 40) 2^-53 =
+4e-14; complex64 inputs, the two transforms of 12 and 10 points (16 stages)
+and results at 2^-24, doubled for the stages' constants: 2.2e-6.
 """
 import numpy as np
 import pytest
@@ -39,6 +40,25 @@ def _sources(m, nz, rng, kind):
 def _layer_errors(y, want, m, nz):
     d = (np.asarray(y, complex) - want).reshape(m.nx * m.ny * 3, nz)
     return np.linalg.norm(d, axis=0) / np.linalg.norm(want.reshape(m.nx * m.ny * 3, nz), axis=0)
+
+
+@pytest.mark.parametrize("nz,f", [(9, 0.1), (22, 0.1), (24, 10.0), (35, 1.0), (48, 0.1)])
+@pytest.mark.parametrize("kind", ["one layer", "falling"])
+@pytest.mark.parametrize("entry", ["c128", "ds"])
+def test_every_layer_in_complex128(egx_ctx, nz, f, kind, entry):
+    m, om, G = _case(egx_ctx, nz, f, nz)
+    g = egx_ctx.green_upload(G, m.nx, m.ny, nz)
+    try:
+        egx_ctx.op_prepare(g, om.zeta, om.zeta0, m.layer_thickness, op.OP_A)
+        rng = np.random.default_rng(nz)
+        xs = [_sources(m, nz, rng, kind), _sources(m, nz, rng, "falling")]
+        apply = egx_ctx.op_apply if entry == "c128" else egx_ctx.op_apply_ds
+        y = apply(np.concatenate(xs), nrhs=2).reshape(2, -1)
+        for i in range(2):
+            err = _layer_errors(y[i], op.apply(G, om, xs[i], op.OP_A), m, nz)
+            assert err.max() < 4e-14, (i, err)
+    finally:
+        g.free()
 
 
 @pytest.mark.parametrize("nz,f", [(9, 0.1), (22, 0.1), (24, 10.0), (35, 1.0), (47, 0.1)])

@@ -25,14 +25,16 @@
 // of split operands takes three MMAs (hi.hi + hi.lo + lo.hi), which keeps
 // complex64 accuracy.
 //
-// Four kernels, one CTA per SM looping over stored points, the offsets of
-// each warp's A fragments held in registers (built once). The -A^T blocks
-// (z rows, x|y columns) take their sign on the B values.
+// Four kernels, one CTA per SM (k_contract_ws with one source two, where they
+// fit: Ws::PER_SM) looping over stored points, the offsets of each warp's A
+// fragments held in registers (built once). The -A^T blocks (z rows, x|y
+// columns) take their sign on the B values.
 //  * k_contract_ws<NZ, NR> (built in, for the two right-hand sides of a
-//    stacked solve of both polarisations and for one): FP16 m16n8k16 with A
-//    fragments straight from the split entries, work split by role -- one
-//    warp per 16-row tile over all column tiles, two warps splitting the next
-//    point's right-hand sides, one producer lane (see the kernel).
+//    stacked solve of both polarisations and for one): A fragments straight
+//    from the split entries (FP16 m16n8k16; one source TF32 m16n8k8), work
+//    split by role -- one warp per 16-row tile over all column tiles, two
+//    warps splitting the next point's right-hand sides, one producer lane (see
+//    the kernel).
 //  * k_contract_sh<NZ> (two; the tuner's variant 2): the same products with
 //    12 warps in lockstep, 3 row groups x 4 column groups, partial sums per
 //    row tile met in shared memory and added by the warps with the fewest
@@ -102,6 +104,12 @@ __device__ __forceinline__ void split(float a, uint32_t &hi, uint32_t &lo) {
 __device__ __forceinline__ void split_rn(float a, uint32_t &hi, uint32_t &lo) {
     hi = tf32_hi(__float_as_uint(a));
     lo = tf32_hi(__float_as_uint(a - __uint_as_float(hi)));
+}
+
+// the same by conversions, which keep a NaN
+__device__ __forceinline__ void split_tf32(float a, uint32_t &hi, uint32_t &lo) {
+    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(hi) : "f"(a));
+    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(lo) : "f"(a - __uint_as_float(hi)));
 }
 
 // 2^(top - e) with 2^(e-1) <= m < 2^e for a normal m > 0, the exponent
@@ -1019,16 +1027,24 @@ __global__ void __launch_bounds__(Sh<NZ>::THREADS, 1)
     }
 }
 
-// k_contract_ws<NZ, NR>: the FP16 split contraction of NR = 1 or 2 sources
+// k_contract_ws<NZ, NR>: the split contraction of NR = 1 or 2 sources
 // with its work split by role, so that the phases of one point overlap the
 // products of another instead of running in lockstep behind block barriers.
 //  * MMA warps, one per row tile (MT of them): every k tile of their tile,
 //    12 products per k tile as in k_contract_sh, accumulators alternating
 //    by k tile; the output leaves from the accumulators (no partial sums).
 //    With one source the eight columns are the real and imaginary parts of
-//    its four points, Gr [Xr | Xi] and Gi [Xr | Xi]: six products per k
-//    tile, and lanes two apart exchange half of their sums, so that each
-//    finishes one row.
+//    its four points, Gr [Xr | Xi] and Gi [Xr | Xi], and lanes two apart
+//    exchange half of their sums, so that each finishes one row. Its products
+//    are TF32 m16n8k8, twelve per k tile: an entry's FP16 parts are TF32 values
+//    as they are, and each value of the right-hand side is split by itself
+//    over the whole FP32 range, so that a layer's share does not lose bits to
+//    a larger one of its column. (FP16 parts under one scale per column, as
+//    for two sources, took 110 us at 128x128x32 instead of 133, and had no bit
+//    left 2^-38 below the column's largest.) The products of low parts have
+//    accumulators of their own, since the tensor cores' accumulators truncate:
+//    2-norm error of an apply against 64 bits 3.2e-8..3.6e-8 where
+//    k_contract_sb's is 3.6e-8..4.4e-8.
 //  * two split warps: load the right-hand sides of a point from global
 //    memory (the Green stage carries no right-hand sides), take one scale
 //    per column over all its rows, split into FP16 fragments in a double
@@ -1038,14 +1054,18 @@ __global__ void __launch_bounds__(Sh<NZ>::THREADS, 1)
 // Hand-offs are mbarriers; every wait is bounded, and a wait that gives up
 // records EGX_ERR_TIMEOUT and raises a block-wide abort flag that ends every
 // role's loop within one poll.
+// one source: the scaled entries of the copy are below 2^15, its right-hand
+// side is taken down by as much
+constexpr float kUp = 32768.f;
+
 template <int NZ, int NR>
 struct Ws {
     static constexpr int R = 3 * NZ, MT = R / 16, KT = R / 16, BS = Sh<NZ>::BS;
     static constexpr int NSPLIT = 2, PRODUCER = MT + NSPLIT, THREADS = 32 * (MT + NSPLIT + 1);
     static constexpr int KPS = (KT + NSPLIT - 1) / NSPLIT;  // k tiles per split warp
     static constexpr uint32_t G_BYTES = BS * 8u;
-    // [KT][Xr, Xi][32 lanes] uint4, or [KT][32 lanes] of [Xr | Xi]
-    static constexpr uint32_t BF_BYTES = KT * NR * 32u * 16u;
+    // [KT][Xr, Xi][32 lanes] uint4, or [KT][high, low][32 lanes] of [Xr | Xi]
+    static constexpr uint32_t BF_BYTES = KT * 2u * 32u * 16u;
     static constexpr uint32_t OFF_BF = 2 * G_BYTES, OFF_INV = OFF_BF + 2 * BF_BYTES;
     static constexpr uint32_t OFF_MAX = OFF_INV + 2u * 8u * 4u;
     static constexpr uint32_t SMEM = OFF_MAX + 2u * NSPLIT * 8u * 4u;
@@ -1153,11 +1173,50 @@ __global__ void __launch_bounds__(Ws<NZ, NR>::THREADS, Ws<NZ, NR>::PER_SM)
             const uint2 *Gq = reinterpret_cast<const uint2 *>(smem + s * P::G_BYTES);
             const uint4 *bfr = BFRAG + (size_t)s * (P::BF_BYTES / 16) + lane;
             // T1 = Gr Xr, T2 = Gi Xi, T3 = Gr Xi, T4 = Gi Xr, even and odd k
-            // tiles; one source: T1 = Gr [Xr | Xi], T2 = Gi [Xr | Xi]
+            // tiles; one source: T1 = Gr [Xr | Xi], T2 = Gi [Xr | Xi], high
+            // products and the others
             constexpr int NT = 2 * NR;
             float acc[2][NT][4];
+            if constexpr (NR == 1) {
 #pragma unroll
-            for (int kt = 0; kt < KT; kt++) {
+                for (int j = 0; j < 16; j++) (&acc[0][0][0])[j] = 0.f;
+#pragma unroll
+                for (int kt = 0; kt < KT; kt++) {
+                    const uint32_t flip = (zrows && (16 * kt) / NZ < 2) ? 0x80000000u : 0u;
+                    // rows 2t, 2t + 1 (first step), 2t + 8, 2t + 9 (second)
+                    const uint4 bh = bfr[(2 * kt) * 32], bl = bfr[(2 * kt + 1) * 32];
+                    const uint32_t hi[4] = {bh.x ^ flip, bh.y ^ flip, bh.z ^ flip, bh.w ^ flip};
+                    const uint32_t lo[4] = {bl.x ^ flip, bl.y ^ flip, bl.z ^ flip, bl.w ^ flip};
+                    const uint32_t t0 = tab[2 * kt], t1 = tab[2 * kt + 1];
+                    const uint32_t ent[4] = {t0 & 0xffffu, t0 >> 16, t1 & 0xffffu, t1 >> 16};
+#pragma unroll
+                    for (int st = 0; st < 2; st++) {
+                        // [Gr hi, Gr lo, Gi hi, Gi lo][a0..a3]: rows g, g + 8 of
+                        // the first column, of the second
+                        uint32_t af[4][4];
+#pragma unroll
+                        for (int e = 0; e < 2; e++) {
+                            const uint32_t off = ent[2 * st + e] & 0x7fffu, nb = (ent[2 * st + e] & 0x8000u) ? 4u : 1u;
+#pragma unroll
+                            for (int c = 0; c < 2; c++) {
+                                const uint2 u = Gq[c ? off ^ nb : off];
+                                const float2 h = __half22float2(*reinterpret_cast<const __half2 *>(&u.x));
+                                const float2 l = __half22float2(*reinterpret_cast<const __half2 *>(&u.y));
+                                af[0][2 * c + e] = __float_as_uint(h.x), af[1][2 * c + e] = __float_as_uint(l.x);
+                                af[2][2 * c + e] = __float_as_uint(h.y), af[3][2 * c + e] = __float_as_uint(l.y);
+                            }
+                        }
+#pragma unroll
+                        for (int j = 0; j < 2; j++) mma_tf32(acc[0][j], af[2 * j], hi[2 * st], hi[2 * st + 1]);
+#pragma unroll
+                        for (int j = 0; j < 2; j++) mma_tf32(acc[1][j], af[2 * j], lo[2 * st], lo[2 * st + 1]);
+#pragma unroll
+                        for (int j = 0; j < 2; j++) mma_tf32(acc[1][j], af[2 * j + 1], hi[2 * st], hi[2 * st + 1]);
+                    }
+                }
+            }
+#pragma unroll
+            for (int kt = 0; kt < KT && NR == 2; kt++) {
                 const uint32_t flip = (zrows && (16 * kt) / NZ < 2) ? 0x80008000u : 0u;
                 // B fragments [Xr, Xi][hi b0, hi b1, lo b0, lo b1]; the sign
                 // flips both FP16 halves (the split commutes with it)
@@ -1185,8 +1244,8 @@ __global__ void __launch_bounds__(Ws<NZ, NR>::THREADS, Ws<NZ, NR>::PER_SM)
                 }
                 float (*ac)[4] = acc[kt & 1];
                 // A part (high) and B operand of product j
-                auto ai = [](int j) { return NR == 1 ? 2 * j : ((j == 0 || j == 2) ? 0 : 2); };
-                auto bi = [](int j) { return NR == 1 ? 0 : ((j == 0 || j == 3) ? 0 : 1); };
+                auto ai = [](int j) { return (j == 0 || j == 2) ? 0 : 2; };
+                auto bi = [](int j) { return NR == 1 || j == 0 || j == 3 ? 0 : 1; };
 #pragma unroll
                 for (int j = 0; j < NT; j++) {
                     if (kt < 2) mma_f16_zero(ac[j], af[ai(j)], bf[bi(j)][0], bf[bi(j)][1]);
@@ -1198,7 +1257,7 @@ __global__ void __launch_bounds__(Ws<NZ, NR>::THREADS, Ws<NZ, NR>::PER_SM)
                 for (int j = 0; j < NT; j++) mma_f16(ac[j], af[ai(j) + 1], bf[bi(j)][0], bf[bi(j)][1]);
             }
             // undo the scales of accumulator columns 2t and 2t + 1
-            const float inv0 = INV[s * 8 + 2 * t], inv1 = INV[s * 8 + 2 * t + 1];
+            const float inv0 = NR == 1 ? ginv * kUp : INV[s * 8 + 2 * t], inv1 = NR == 1 ? inv0 : INV[s * 8 + 2 * t + 1];
             mbar_arrive(b_sempty + 8 * s);
             mbar_arrive(b_bempty + 8 * s);
             const int a = (int)((unsigned)q / (unsigned)(ny + 1)), bq = q - a * (ny + 1);
@@ -1280,6 +1339,7 @@ __global__ void __launch_bounds__(Ws<NZ, NR>::THREADS, Ws<NZ, NR>::PER_SM)
                 }
             }
             if (it >= 2 && !ws_wait_warp(b_bempty + 8 * s, par ^ 1u, abort, err)) break;
+            uint4 *bfw = BFRAG + (size_t)s * (P::BF_BYTES / 16) + lane;
             float m = 0.f;
 #pragma unroll
             for (int i = 0; i < P::KPS; i++) {
@@ -1300,6 +1360,23 @@ __global__ void __launch_bounds__(Ws<NZ, NR>::THREADS, Ws<NZ, NR>::PER_SM)
                     m = fmaxf(m, fmaxf(fmaxf(fabsf(xv[i][h].x), fabsf(xv[i][h].y)),
                                        fmaxf(fabsf(xv[i][h].z), fabsf(xv[i][h].w))));
             }
+            if constexpr (NR == 1) {
+                const bool im = g >= 4;
+#pragma unroll
+                for (int i = 0; i < P::KPS; i++) {
+                    const int kt = hh + P::NSPLIT * i;
+                    if (kt >= KT) continue;
+                    uint4 h, l;
+                    split_tf32((im ? xv[i][0].y : xv[i][0].x) / kUp, h.x, l.x);
+                    split_tf32((im ? xv[i][0].w : xv[i][0].z) / kUp, h.y, l.y);
+                    split_tf32((im ? xv[i][1].y : xv[i][1].x) / kUp, h.z, l.z);
+                    split_tf32((im ? xv[i][1].w : xv[i][1].z) / kUp, h.w, l.w);
+                    bfw[(2 * kt) * 32] = h;
+                    bfw[(2 * kt + 1) * 32] = l;
+                }
+                mbar_arrive(b_bfull + 8 * s);
+                continue;
+            }
             // one scale per column over all its rows: the split warps'
             // maxima meet in shared memory
             m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 1));
@@ -1311,23 +1388,12 @@ __global__ void __launch_bounds__(Ws<NZ, NR>::THREADS, Ws<NZ, NR>::PER_SM)
 #pragma unroll
             for (int h = 0; h < P::NSPLIT; h++) mc = fmaxf(mc, CMAX[(s * P::NSPLIT + h) * 8 + g]);
             const float scB = pow2_scale(mc, 13);
-            uint4 *bfw = BFRAG + (size_t)s * (P::BF_BYTES / 16) + lane;
 #pragma unroll
             for (int i = 0; i < P::KPS; i++) {
                 const int kt = hh + P::NSPLIT * i;
                 if (kt >= KT) continue;
                 // [Xr, Xi] x [hi b0, hi b1, lo b0, lo b1]
                 uint4 fr, fi;
-                if constexpr (NR == 1) {
-                    const bool im = g >= 4;
-#pragma unroll
-                    for (int h = 0; h < 2; h++) {
-                        const float u = im ? xv[i][h].y : xv[i][h].x, w = im ? xv[i][h].w : xv[i][h].z;
-                        split_h2(u * scB, w * scB, h ? fr.y : fr.x, h ? fr.w : fr.z);
-                    }
-                    bfw[kt * 32] = fr;
-                    continue;
-                }
                 split_h2(xv[i][0].x * scB, xv[i][0].z * scB, fr.x, fr.z);
                 split_h2(xv[i][1].x * scB, xv[i][1].z * scB, fr.y, fr.w);
                 split_h2(xv[i][0].y * scB, xv[i][0].w * scB, fi.x, fi.z);
@@ -1404,8 +1470,8 @@ void launch_nz(float2 *buf, const float2 *G, const OpDims &d, int *err, cudaStre
     // contract_variant: 1 k_contract_sb3 (TF32 split), 2 k_contract_sh
     // (FP16 split, all warps in lockstep), 0 the built-in choice:
     // k_contract_ws (FP16 split by role: 1.110 against 1.293 ms per
-    // two-source launch at 256x256x48; one source at 128x128x32 110 us,
-    // 0.9 of the copy bandwidth, against 254 of k_contract_sb)
+    // two-source launch at 256x256x48; one source at 128x128x32 133 us,
+    // 0.74 of the copy bandwidth, against 254 of k_contract_sb)
     const int v = d.contract_variant;
     for (int r0 = 0; r0 < d.nrhs;) {
         if (d.nrhs - r0 >= 2) {

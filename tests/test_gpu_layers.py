@@ -5,7 +5,9 @@ different size, and the small ones are to be as accurate as the large ones.
 Tolerances, of each layer's own 2-norm: complex128 both sides round at 2^-53,
 at most 300 terms and 40 operations of the transforms, (300 + 40) 2^-53 =
 4e-14; complex64 inputs, the two transforms of 12 and 10 points (16 stages)
-and results at 2^-24, doubled for the stages' constants: 2.2e-6.
+and results at 2^-24, doubled for the stages' constants: 2.2e-6; the sub-block
+layout of complex64 keeps 22 bits of an operand: 2e-5, as in the other tests of
+its kernels.
 """
 import numpy as np
 import pytest
@@ -76,5 +78,39 @@ def test_every_layer_in_complex64(egx_ctx, nz, f, kind):
             for i in range(nrhs):
                 err = _layer_errors(y[i], op.apply(G, om, xs[i].astype(complex), op.OP_A), m, nz)
                 assert err.max() < 2.2e-6, (nrhs, i, err)
+    finally:
+        g.free()
+
+
+@pytest.mark.parametrize("nz", [16, 32, 48])
+def test_every_layer_of_one_source_in_the_subblock_layout(egx_ctx, nz):
+    """Layers without coupling: each one's response is its own source's, of
+    whatever size that is beside the others."""
+    m, om, G = _case(egx_ctx, nz, 0.1, nz)
+    tr, rc = np.meshgrid(np.arange(nz), np.arange(nz), indexing="ij")
+    up = rc <= tr
+    G = {c: v * ((rc == tr).reshape(-1) if c in ("xz", "yz") else (rc == tr)[up]) for c, v in G.items()}
+    g = egx_ctx.green_upload(G, m.nx, m.ny, nz, precision=egx.PREC_MIXED)
+    try:
+        egx_ctx.op_prepare(g, om.zeta, om.zeta0, m.layer_thickness, op.OP_A)
+        x = _sources(m, nz, np.random.default_rng(nz), "falling").astype(np.complex64)
+        err = _layer_errors(egx_ctx.op_apply_c64(x), op.apply(G, om, x.astype(complex), op.OP_A), m, nz)
+        assert err.max() < 2e-5, err
+    finally:
+        g.free()
+
+
+@pytest.mark.parametrize("nz", [9, 16, 32])
+def test_one_complex64_source_keeps_what_is_not_finite(egx_ctx, nz):
+    m, om, G = _case(egx_ctx, nz, 0.1, nz)
+    g = egx_ctx.green_upload(G, m.nx, m.ny, nz, precision=egx.PREC_MIXED)
+    try:
+        egx_ctx.op_prepare(g, om.zeta, om.zeta0, m.layer_thickness, op.OP_A)
+        x = np.ones(m.nx * m.ny * 3 * nz, np.complex64)
+        assert np.isfinite(egx_ctx.op_apply_c64(x)).all()
+        for bad in (np.nan, np.inf, 1j * np.inf):
+            xb = x.copy()
+            xb[len(x) // 2] = bad
+            assert not np.isfinite(egx_ctx.op_apply_c64(xb)).any()
     finally:
         g.free()

@@ -193,7 +193,7 @@ __device__ __forceinline__ double value(Sum s, int e) {
         p = -__clzll((long long)l);
         m = l << -p;
     }
-    return round_f64(m, p + e, neg);
+    return round_f64(m, p + e, neg ? 0x80000000u : 0u);
 }
 
 // The kernel's shared memory. Rows and columns are counted with nz rounded up

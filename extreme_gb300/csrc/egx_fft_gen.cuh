@@ -292,19 +292,23 @@ __device__ __forceinline__ long long fix_in(double x, int E) {
     const long long sg = (long long)((int)hi >> 31);
     return (long long)((v ^ (unsigned long long)sg) - (unsigned long long)sg);
 }
-// v 2^e rounded to nearest, ties to even; below the normal range 0
-__device__ __forceinline__ double fix_out(long long v, int e) {
+// v 2^e rounded to nearest, ties to even, v a number of a column under exponent
+// E. tiny: a result can lie below the normal range (E < kTiny); e is then kUp
+// more than it is, and a product by a power of two rounds once more.
+constexpr int kTiny = 64, kUp = 128;
+__device__ __forceinline__ double fix_out(long long v, int e, bool tiny) {
     const uint32_t sign = (uint32_t)(v >> 32) & 0x80000000u;
     const unsigned long long u = (unsigned long long)(v < 0 ? -v : v);
     const int lz = __clzll((long long)u);
     unsigned long long m = u << lz;
     m += 0x3ffull + ((m >> 11) & 1);
     const bool carry = m < 0x8000000000000000ull;
-    int be = 1023 + 63 - lz + e + (carry ? 1 : 0);
-    if (u == 0 || be <= 0) return __hiloint2double((int)sign & (u == 0 ? 0 : -1), 0);
+    const int be = 1023 + 63 - lz + e + (carry ? 1 : 0);
+    if (u == 0) return 0.0;
     const unsigned long long f = carry ? 0 : ((m >> 11) & 0xfffffffffffffull);
     if (be >= 2047) return __hiloint2double((int)(sign | 0x7ff00000u), 0);
-    return __hiloint2double((int)(sign | ((uint32_t)be << 20) | (uint32_t)(f >> 32)), (int)(uint32_t)f);
+    const double r = __hiloint2double((int)(sign | ((uint32_t)be << 20) | (uint32_t)(f >> 32)), (int)(uint32_t)f);
+    return tiny ? r * 2.938735877055719e-39 : r;  // 2^-kUp
 }
 
 __device__ __forceinline__ int fft_bexp(double2 v) {
@@ -393,9 +397,10 @@ __device__ __forceinline__ void gen_last(const typename FftArith<T>::type::V *S,
 #pragma unroll
         for (int r = 0; r < R; r++) {
             if constexpr (sizeof(T) == sizeof(double)) {
-                const int e = E - 1081 + p.sh_sum;
-                const bool bad = E == 2047;
-                const double a = bad ? (double)NAN : fix_out(v[r].x, e), b = bad ? (double)NAN : fix_out(v[r].y, e);
+                const bool bad = E == 2047, tiny = E < kTiny;
+                const int e = E - 1081 + p.sh_sum + (tiny ? kUp : 0);
+                const double a = bad ? (double)NAN : fix_out(v[r].x, e, tiny);
+                const double b = bad ? (double)NAN : fix_out(v[r].y, e, tiny);
                 store(j + r * nr, swap ? make_double2(b, a) : make_double2(a, b));
             } else {
                 store(j + r * nr, swap ? mk<T>(v[r].y, v[r].x) : v[r]);

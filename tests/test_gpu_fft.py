@@ -44,3 +44,21 @@ def test_fft2d_nonfinite_and_zero_columns(egx_ctx):
     assert not got[..., 0].any()
     assert not np.isfinite(got[..., 1]).any() and not np.isfinite(got[..., 2]).any()
     assert np.array_equal(got[..., 3], want[..., 3])
+
+
+def test_fft2d_of_subnormal_numbers(egx_ctx):
+    """Columns at and below 2^-1022 against the transform of the same columns
+    scaled into the normal range. A result is rounded to units of 2^-1074 after
+    each of the two passes: half a unit per entry, at most 30 of them summed by
+    the second pass, in both parts: (30 + 1) / 2 sqrt(2) < 24 units."""
+    rng = np.random.default_rng(5)
+    a = rng.standard_normal((30, 28, 4)) + 1j * rng.standard_normal((30, 28, 4))
+    down = np.array([1040, 1024, 1018, 1060])
+    unit = np.ldexp(1.0, -1074)
+    x = np.ldexp(a.real, -down) + 1j * np.ldexp(a.imag, -down)
+    back = np.ldexp(x.real, down - 8) + 1j * np.ldexp(x.imag, down - 8)  # exact
+    want = np.fft.fft2(back, axes=(0, 1))
+    got = egx_ctx.fft2d(x.copy(), -1)
+    for c in range(4):
+        g = np.ldexp(got[..., c].real, down[c] - 8) + 1j * np.ldexp(got[..., c].imag, down[c] - 8)
+        assert np.abs(g - want[..., c]).max() < 24 * np.ldexp(unit, down[c] - 8) + TOL * np.linalg.norm(want[..., c])

@@ -63,6 +63,24 @@ def test_every_layer_in_complex128(egx_ctx, nz, f, kind, entry):
         g.free()
 
 
+def test_subnormal_vector_in_complex128(egx_ctx):
+    """2^-1040 times a vector gives 2^-1040 times the result, to what rounding
+    to units of 2^-1074 leaves: half a unit in each of ten steps, summed over
+    120 spectral points by an operator of norm below three, 1,800 units."""
+    nz = 9
+    m, om, G = _case(egx_ctx, nz, 0.1, nz)
+    g = egx_ctx.green_upload(G, m.nx, m.ny, nz)
+    try:
+        egx_ctx.op_prepare(g, om.zeta, om.zeta0, m.layer_thickness, op.OP_A)
+        rng = np.random.default_rng(1)
+        x = rng.standard_normal(m.nx * m.ny * 3 * nz) + 1j * rng.standard_normal(m.nx * m.ny * 3 * nz)
+        y, small = egx_ctx.op_apply(x), egx_ctx.op_apply(np.ldexp(x.real, -1040) + 1j * np.ldexp(x.imag, -1040))
+        d = np.ldexp(small.real, 1040) + 1j * np.ldexp(small.imag, 1040) - y
+        assert np.abs(d).max() < 1800 * 2.0 ** (1040 - 1074)
+    finally:
+        g.free()
+
+
 @pytest.mark.parametrize("nz,f", [(9, 0.1), (22, 0.1), (24, 10.0), (35, 1.0), (47, 0.1)])
 @pytest.mark.parametrize("kind", ["one layer", "falling"])
 def test_every_layer_in_complex64(egx_ctx, nz, f, kind):

@@ -270,6 +270,7 @@ GreenModel green_model(const egx_model *model, double omega) {
 
 void ensure_twiddles(egx_ctx *ctx, int n0, int n1) {
     if (ctx->tw_n0 == n0 && ctx->tw_n1 == n1) return;
+    ctx->tw_n0 = ctx->tw_n1 = 0;  // no tables until all four are there
     ctx->p0 = make_fft_plan(n0);
     ctx->p1 = make_fft_plan(n1);
     upload_table(ctx->tw0_64, fft_table64(n0), ctx->stream);
@@ -307,6 +308,7 @@ void prepare_device(egx_ctx *ctx, egx_green *g, const double *dz, int type) {
         bwd[k] = sc;
     }
     const long ncell = (long)nx * ny;
+    ctx->g = nullptr;  // no operator until all of it is there
     ctx->r64.ensure(ncell * nz * sizeof(double2));
     ctx->fwd64.ensure(nz * sizeof(double2));
     ctx->bwd64.ensure(nz * sizeof(double2));
@@ -1048,6 +1050,14 @@ int egx_learned_inject_nonfinite(egx_ctx *ctx, int count) {
     EGX_GUARD(ctx, {
         EGX_CHECK(count >= 0, EGX_ERR_INVALID, "injection count must be >= 0");
         ctx->learned_inject = count;
+    });
+}
+
+int egx_inject_alloc_failure(egx_ctx *ctx, int n) {
+    if (!ctx) return EGX_ERR_INVALID;
+    EGX_GUARD(ctx, {
+        EGX_CHECK(n >= 0, EGX_ERR_INVALID, "allocation count must be >= 0");
+        alloc_failure() = n;
     });
 }
 

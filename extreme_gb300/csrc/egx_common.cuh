@@ -150,10 +150,19 @@ inline std::atomic<long> &device_allocations() {
     return n;
 }
 
+// Test hook (egx_inject_alloc_failure): the n-th allocation of the calling
+// thread from now fails; 0, none.
+inline int &alloc_failure() {
+    static thread_local int n = 0;
+    return n;
+}
+
 // cudaMalloc that counts the allocation; throws EGX_ERR_OOM (with `what`)
 // when it fails.
 inline void *device_alloc(size_t bytes, const char *what) {
     void *p = nullptr;
+    int &n = alloc_failure();
+    if (n > 0 && --n == 0) throw Error(EGX_ERR_OOM, std::string(what) + ": allocation failure asked for");
     cudaError_t e = cudaMalloc(&p, bytes);
     if (e != cudaSuccess)
         throw Error(EGX_ERR_OOM, std::string(what) + ": cudaMalloc of " + std::to_string(bytes) +

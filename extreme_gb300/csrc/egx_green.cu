@@ -864,15 +864,19 @@ X *dev_upload(DevBuf &b, const std::vector<X> &v, cudaStream_t s) {
     return b.as<X>();
 }
 
-// the workspace's FFT tables of lengths n0 and n1, kept while they fit
+// The workspace's FFT tables of lengths n0 and n1, kept while they fit. What is
+// kept has no key while it is replaced: an allocation that fails in between
+// leaves nothing that a later build would take for its own.
 void fft_tables64(GreenWorkspace &w, int n0, int n1, cudaStream_t s) {
     if (w.n64[0] == n0 && w.n64[1] == n1) return;
+    w.n64[0] = w.n64[1] = 0;
     dev_upload(w.tw0, fft_table64(n0), s);
     dev_upload(w.tw1, fft_table64(n1), s);
     w.n64[0] = n0, w.n64[1] = n1;
 }
 void fft_tables32(GreenWorkspace &w, int n0, int n1, cudaStream_t s) {
     if (w.n32[0] == n0 && w.n32[1] == n1) return;
+    w.n32[0] = w.n32[1] = 0;
     dev_upload(w.tw0_32, fft_table32(n0), s);
     dev_upload(w.tw1_32, fft_table32(n1), s);
     w.n32[0] = n0, w.n32[1] = n1;
@@ -1750,6 +1754,7 @@ void build_level_green(const GreenModel &m, int n_hankels, double z, double shx,
         std::vector<double> key = {(double)m.nx, (double)m.ny, m.dx, m.dy, shx, shy};
         key.insert(key.end(), radii.begin(), radii.end());
         if (key != w.lkey[form][kind]) {
+            w.lkey[form][kind].clear();
             std::vector<std::vector<int>> rp;
             std::vector<std::vector<Term>> tt;
             level_terms(m, radii, shx, shy, kind, ncomp, rp, tt);

@@ -32,6 +32,7 @@ EXPORTS = [
     "egx_wait_selftest",
     "egx_net_create", "egx_net_free", "egx_net_size", "egx_net_params", "egx_net_set_model", "egx_net_set_models", "egx_net_loss_grad",
     "egx_net_adam", "egx_net_use_tcgen05", "egx_net_apply", "egx_learned_stats", "egx_learned_inject_nonfinite",
+    "egx_inject_alloc_failure",
 ]
 
 # kernel kinds of egx_profile_read
@@ -143,6 +144,7 @@ def load(path=None):
     lib.egx_net_apply.argtypes = [vp, vp, vp, vp, i, i]
     lib.egx_learned_stats.argtypes = [vp, C.POINTER(C.c_long), C.POINTER(C.c_long)]
     lib.egx_learned_inject_nonfinite.argtypes = [vp, i]
+    lib.egx_inject_alloc_failure.argtypes = [vp, i]
     lib.egx_profile.argtypes = [vp, i]
     lib.egx_profile_kinds.argtypes = [vp, C.c_uint]
     lib.egx_profile_read.argtypes = [vp, i, C.POINTER(C.c_long), C.POINTER(C.c_double)]
@@ -471,6 +473,11 @@ class Context:
         uses, fb = C.c_long(), C.c_long()
         self._check(self.lib.egx_learned_stats(self.h, C.byref(uses), C.byref(fb)))
         return uses.value, fb.value
+
+    def inject_alloc_failure(self, n):
+        """Test hook: the n-th device allocation of this thread from now on
+        fails with ERR_OOM; 0 disarms it."""
+        self._check(self.lib.egx_inject_alloc_failure(self.h, int(n)))
 
     def learned_inject_nonfinite(self, count):
         """Test hook: the next `count` learned-preconditioner outputs get a

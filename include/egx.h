@@ -260,6 +260,12 @@ int egx_learned_stats(egx_ctx *ctx, long *uses, long *fallbacks);
  * non-finite norm stops at once as not converged. count 0 disarms it. */
 int egx_learned_inject_nonfinite(egx_ctx *ctx, int count);
 
+/* Failure-injection hook for tests (no reference counterpart): the n-th device
+ * allocation that the calling thread makes from now on fails with EGX_ERR_OOM,
+ * as if the memory had run out (nothing is asked of the device). n 0 disarms
+ * it. */
+int egx_inject_alloc_failure(egx_ctx *ctx, int n);
+
 /* Failure-detection check (no reference counterpart): one kernel waits,
  * through the bounded wait that every TMA-fed kernel uses, on a shared-memory
  * barrier that nothing completes, and gives up after limit_ms (1..2000).

@@ -448,12 +448,12 @@ __global__ void k_term_values(Term *terms, long n, const double *__restrict__ ra
 // terms are a run of consecutive pieces, so a value's terms of a run are at
 // known places; the runs are found first. (Next to the source a cell has
 // hundreds of terms in them.) A cell has two faces in each direction, each in
-// at most two parts: eight runs. First the counts (WRITE false: ptr[cell +
-// 1]), then, with the rows' starts in ptr, the nodes.
+// at most two parts: eight runs; more raise `over`. First the counts (WRITE
+// false: ptr[cell + 1]), then, with the rows' starts in ptr, the nodes.
 constexpr int kRuns = 8;
 template <bool WRITE>
 __global__ void k_term_nodes(const int *__restrict__ rowptr, const Term *__restrict__ terms, int ncell, int nsrc,
-                             int nrad, int *ptr, Node *__restrict__ nodes) {
+                             int nrad, int *ptr, Node *__restrict__ nodes, int *over) {
     const int cell = (int)(((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
     if (cell >= ncell) return;
     const int e0 = rowptr[cell], e1 = rowptr[cell + 1];
@@ -476,6 +476,7 @@ __global__ void k_term_nodes(const int *__restrict__ rowptr, const Term *__restr
         if (first && at < kRuns) start[at] = e;
         runs += __popc(m);
     }
+    if (!WRITE && lane == 0 && runs > kRuns) *over = 1;
     runs = min(runs, kRuns);
     if (lane == 0) start[runs] = e1;
     __syncwarp();
@@ -1274,17 +1275,19 @@ void make_nodes(GreenWorkspace &w, GreenWorkspace::CellLists &cl, const std::vec
     const long n = (long)terms.size();
     const int *row = dev_upload(w.d_trow, rowptr, s);
     Term *t = dev_upload(w.d_terms, terms, s);
-    cl.rowptr.ensure(rowptr.size() * sizeof(int));
-    int *ptr = cl.rowptr.as<int>();
+    cl.rowptr.ensure((rowptr.size() + 1) * sizeof(int));
+    int *ptr = cl.rowptr.as<int>(), *over = ptr + ncell + 1;
+    EGX_CUDA(cudaMemsetAsync(over, 0, sizeof(int), s));
     const unsigned warps = (unsigned)(((long)ncell * 32 + 255) / 256);
     k_term_values<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(t, n, radii_dev);
-    k_term_nodes<false><<<warps, 256, 0, s>>>(row, t, ncell, nsrc, nrad, ptr, nullptr);
+    k_term_nodes<false><<<warps, 256, 0, s>>>(row, t, ncell, nsrc, nrad, ptr, nullptr, over);
     k_running_sum<<<1, 1024, 0, s>>>(ptr, ncell);
-    int total = 0;
-    EGX_CUDA(cudaMemcpyAsync(&total, ptr + ncell, sizeof(int), cudaMemcpyDeviceToHost, s));
+    int last[2] = {};  // all nodes; whether a cell has more runs than its faces can make
+    EGX_CUDA(cudaMemcpyAsync(last, ptr + ncell, sizeof last, cudaMemcpyDeviceToHost, s));
     EGX_CUDA(cudaStreamSynchronize(s));
-    cl.terms.ensure(std::max(1, total) * sizeof(Node));
-    k_term_nodes<true><<<warps, 256, 0, s>>>(row, t, ncell, nsrc, nrad, ptr, cl.terms.as<Node>());
+    EGX_CHECK(!last[1], EGX_ERR_MODEL, "a cell's face terms make more runs than its faces");
+    cl.terms.ensure((size_t)std::max(1, last[0]) * sizeof(Node));
+    k_term_nodes<true><<<warps, 256, 0, s>>>(row, t, ncell, nsrc, nrad, ptr, cl.terms.as<Node>(), over);
     EGX_CUDA(cudaGetLastError());
     if (launches) *launches += 4;
 }

@@ -9,35 +9,12 @@ namespace egx {
 
 constexpr int kThreads = 256;
 
-template <typename T> struct Acc { typedef T type; };
-
-__device__ __forceinline__ double2 warp_sum2(double2 v) {
-    for (int o = 16; o > 0; o >>= 1) {
-        v.x += __shfl_down_sync(0xffffffffu, v.x, o);
-        v.y += __shfl_down_sync(0xffffffffu, v.y, o);
-    }
-    return v;
-}
 __device__ __forceinline__ double warp_sum(double v) {
     for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
     return v;
 }
 
 // Block-wide sum; result valid in thread 0.
-__device__ double2 block_sum2(double2 v) {
-    __shared__ double2 red[32];
-    v = warp_sum2(v);
-    int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    __syncthreads();
-    if (lane == 0) red[wid] = v;
-    __syncthreads();
-    if (wid == 0) {
-        int nw = (blockDim.x + 31) >> 5;
-        v = lane < nw ? red[lane] : make_double2(0, 0);
-        v = warp_sum2(v);
-    }
-    return v;
-}
 __device__ double block_sum(double v) {
     __shared__ double red1[32];
     v = warp_sum(v);

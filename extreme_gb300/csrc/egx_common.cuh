@@ -223,10 +223,15 @@ struct DevBuf {
 // previous kernel's end and its writes, then let the next kernel do the same.
 // Every kernel launched with launch_after() calls after_previous() before it
 // touches memory and on every path, so the order of writes is that of plain
-// launches. `bytes`: what the kernel works through. With more than half of the
-// L2 the gap between kernels is nothing and the waiting blocks only take room
-// (four passes and a contraction over 50 MB 205 -> 198 us, over 604 MB 1,776 ->
-// 1,793 us): those are launched plainly.
+// launches. `bytes`: what the kernel works through, the transform buffer of an
+// apply or the columns of a Gram-Schmidt pass. Beyond half of the L2 the gap
+// between kernels is small beside them and the waiting blocks take room, so
+// those are launched plainly. Applies, plain against early: 13 MB 83.1 and
+// 74.7 us, 50 MB 217.6 and 208.1, 64 MB 277.7 and 272.4, 113 MB 467.6 and
+// 461.0; from 150 MB on now one, now the other is ahead (226 MB 725.9 and 716.6
+// in complex64, 2,987 and 3,021 in complex128; 201 MB 809 and 843; 604 MB 1,776
+// and 1,793). Whole solves of 32x32x8 23.4 and 20.4 ms, of 90x75x22 93.3 and
+// 85.7.
 constexpr size_t kEarlyBytes = 64u << 20;
 __device__ __forceinline__ void after_previous() {
     asm volatile("griddepcontrol.wait;" ::: "memory");

@@ -251,7 +251,8 @@ __global__ void __launch_bounds__(MAXT, MINB)
     for (int i = tid; i < MT * KT * 32; i += blockDim.x) {
         const int ln = i & 31, tile = i >> 5, tm = tile / KT, r = 16 * tm + (ln >> 2);
         const int c = 16 * (tile - tm * KT) + 2 * (ln & 3);
-        tab[i] = make_uint4(dig_word(nz, r, c), dig_word(nz, r + 8, c), dig_word(nz, r, c + 8), dig_word(nz, r + 8, c + 8));
+        tab[i] = make_uint4(dig_word(nz, r, c), dig_word(nz, r + 8, c), dig_word(nz, r, c + 8),
+                            dig_word(nz, r + 8, c + 8));
     }
     auto fetch = [&](int q) {  // the point's block; one thread
         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(sbar), "r"(m.point) : "memory");

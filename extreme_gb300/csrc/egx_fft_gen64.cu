@@ -9,9 +9,9 @@ namespace {
 
 // lines whose second half is the parity image of the first (see k_lines_sym_r)
 template <int CLS>
-__global__ void __launch_bounds__(gen_max_threads<double, CLS>(), gen_min_blocks<double, CLS>()) k_lines_sym_g(double2 *buf, long lstride, long estride, int B, int parity,
-                                                     int nstore, const GenPlan p, const double2 *__restrict__ tw,
-                                                     int lbt, int sign) {
+__global__ void __launch_bounds__(gen_max_threads<double, CLS>(), gen_min_blocks<double, CLS>())
+    k_lines_sym_g(double2 *buf, long lstride, long estride, int B, int parity, int nstore, const GenPlan p,
+                  const double2 *__restrict__ tw, int lbt, int sign) {
     extern __shared__ __align__(16) unsigned char smem[];
     const int b = (blockIdx.x << lbt) + (threadIdx.x & ((1 << lbt) - 1));
     const bool bok = b < B;

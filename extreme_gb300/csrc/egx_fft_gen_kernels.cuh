@@ -15,8 +15,9 @@ namespace {
 
 // rx = r x scaled by the forward factors (real), zero-padded, DFT along y
 template <typename T, int CLS>
-__global__ void __launch_bounds__(gen_max_threads<T, CLS>(), gen_min_blocks<T, CLS>()) k_fwd_y_g(const C<T> *__restrict__ x, const OperatorData<T> op, C<T> *__restrict__ buf,
-                                                 const OpDims d, const GenPlan p, const C<T> *__restrict__ tw, int lbt) {
+__global__ void __launch_bounds__(gen_max_threads<T, CLS>(), gen_min_blocks<T, CLS>())
+    k_fwd_y_g(const C<T> *__restrict__ x, const OperatorData<T> op, C<T> *__restrict__ buf, const OpDims d,
+              const GenPlan p, const C<T> *__restrict__ tw, int lbt) {
     extern __shared__ __align__(16) unsigned char smem[];
     after_previous();
     const int i = blockIdx.y, b = (blockIdx.x << lbt) + (threadIdx.x & ((1 << lbt) - 1));
@@ -38,8 +39,9 @@ __global__ void __launch_bounds__(gen_max_threads<T, CLS>(), gen_min_blocks<T, C
 }
 
 template <typename T, int CLS>
-__global__ void __launch_bounds__(gen_max_threads<T, CLS>(), gen_min_blocks<T, CLS>()) k_lines_g(C<T> *buf, long lstride, long estride, int B, int nload, int nstore,
-                                                 const GenPlan p, const C<T> *__restrict__ tw, int lbt, int sign) {
+__global__ void __launch_bounds__(gen_max_threads<T, CLS>(), gen_min_blocks<T, CLS>())
+    k_lines_g(C<T> *buf, long lstride, long estride, int B, int nload, int nstore, const GenPlan p,
+              const C<T> *__restrict__ tw, int lbt, int sign) {
     extern __shared__ __align__(16) unsigned char smem[];
     after_previous();
     const int b = (blockIdx.x << lbt) + (threadIdx.x & ((1 << lbt) - 1));
@@ -54,9 +56,9 @@ __global__ void __launch_bounds__(gen_max_threads<T, CLS>(), gen_min_blocks<T, C
 
 // inverse DFT along y, backward factors (real) and the last step
 template <typename T, int CLS>
-__global__ void __launch_bounds__(gen_max_threads<T, CLS>(), gen_min_blocks<T, CLS>()) k_bwd_y_g(const C<T> *__restrict__ buf, const C<T> *__restrict__ x,
-                                                 const OperatorData<T> op, C<T> *__restrict__ y, const OpDims d,
-                                                 const GenPlan p, const C<T> *__restrict__ tw, int lbt) {
+__global__ void __launch_bounds__(gen_max_threads<T, CLS>(), gen_min_blocks<T, CLS>())
+    k_bwd_y_g(const C<T> *__restrict__ buf, const C<T> *__restrict__ x, const OperatorData<T> op,
+              C<T> *__restrict__ y, const OpDims d, const GenPlan p, const C<T> *__restrict__ tw, int lbt) {
     extern __shared__ __align__(16) unsigned char smem[];
     after_previous();
     const int i = blockIdx.y, b = (blockIdx.x << lbt) + (threadIdx.x & ((1 << lbt) - 1));
@@ -99,7 +101,8 @@ bool gen_fwd_y(const FftPlan &p, const C<T> *x, const OperatorData<T> &op, C<T> 
     auto run = [&](auto cls) {
         constexpr int K = decltype(cls)::value;
         raise_smem_limit((const void *)k_fwd_y_g<T, K>, l.smem);
-        launch_after(buffer_bytes<T>(d), k_fwd_y_g<T, K>, gen_grid(d.B, l.lbt, d.nx), l.threads, l.smem, s, x, op, buf, d, p.gen, tw, l.lbt);
+        launch_after(buffer_bytes<T>(d), k_fwd_y_g<T, K>, gen_grid(d.B, l.lbt, d.nx), l.threads, l.smem, s, x, op, buf,
+                     d, p.gen, tw, l.lbt);
     };
     by_class(p.gen, run);
     return true;
@@ -113,7 +116,8 @@ bool gen_bwd_y(const FftPlan &p, const C<T> *buf, const C<T> *x, const OperatorD
     auto run = [&](auto cls) {
         constexpr int K = decltype(cls)::value;
         raise_smem_limit((const void *)k_bwd_y_g<T, K>, l.smem);
-        launch_after(buffer_bytes<T>(d), k_bwd_y_g<T, K>, gen_grid(d.B, l.lbt, d.nx), l.threads, l.smem, s, buf, x, op, y, d, p.gen, tw, l.lbt);
+        launch_after(buffer_bytes<T>(d), k_bwd_y_g<T, K>, gen_grid(d.B, l.lbt, d.nx), l.threads, l.smem, s, buf, x, op,
+                     y, d, p.gen, tw, l.lbt);
     };
     by_class(p.gen, run);
     return true;
@@ -127,8 +131,8 @@ bool gen_lines(const FftPlan &p, C<T> *buf, int nlines, long lstride, long estri
     auto run = [&](auto cls) {
         constexpr int K = decltype(cls)::value;
         raise_smem_limit((const void *)k_lines_g<T, K>, l.smem);
-        launch_after((size_t)nlines * p.n * B * sizeof(C<T>), k_lines_g<T, K>, gen_grid(B, l.lbt, nlines), l.threads, l.smem, s, buf, lstride, estride, B, nload,
-                     nstore, p.gen, tw, l.lbt, sign);
+        launch_after((size_t)nlines * p.n * B * sizeof(C<T>), k_lines_g<T, K>, gen_grid(B, l.lbt, nlines), l.threads,
+                     l.smem, s, buf, lstride, estride, B, nload, nstore, p.gen, tw, l.lbt, sign);
     };
     by_class(p.gen, run);
     return true;

@@ -502,22 +502,24 @@ template <typename T>
 void VecOps<T>::multi_dot(const C<T> *V, int ncols, const C<T> *w, long n, double2 *dots_dev, const GsScratch &g,
                           cudaStream_t s, const int *live, long long *count) {
     if (sizeof(T) == sizeof(float) && n % 2 == 0 && aligned16(V) && aligned16(w))
-        launch_after((size_t)n * ncols * sizeof(C<T>), k_multi_dot_c2, g.nblocks, kThreads, 0, s, reinterpret_cast<const float4 *>(V), ncols,
-                     reinterpret_cast<const float4 *>(w), n / 2, g.partials, dots_dev, g.counter, live, count);
+        launch_after((size_t)n * ncols * sizeof(C<T>), k_multi_dot_c2, g.nblocks, kThreads, 0, s,
+                     reinterpret_cast<const float4 *>(V), ncols, reinterpret_cast<const float4 *>(w), n / 2,
+                     g.partials, dots_dev, g.counter, live, count);
     else
-        launch_after((size_t)n * ncols * sizeof(C<T>), k_multi_dot<T>, g.nblocks, kThreads, 0, s, V, ncols, w, n, g.partials, dots_dev, g.counter, live,
-                     count);
+        launch_after((size_t)n * ncols * sizeof(C<T>), k_multi_dot<T>, g.nblocks, kThreads, 0, s, V, ncols, w, n,
+                     g.partials, dots_dev, g.counter, live, count);
 }
 template <typename T>
 static void launch_update(const C<T> *V, int ncols, const double2 *dots_dev, C<T> *w, long n, double *norm2_dev,
                           const GsScratch &g, cudaStream_t s, const int *live, const GsControl &gs) {
     double *part = reinterpret_cast<double *>(g.partials);
     if (sizeof(T) == sizeof(float) && n % 2 == 0 && aligned16(V) && aligned16(w))
-        launch_after((size_t)n * ncols * sizeof(C<T>), k_update_norm_c2, g.nblocks, kThreads, 0, s, reinterpret_cast<const float4 *>(V), ncols, dots_dev,
-                     reinterpret_cast<float4 *>(w), n / 2, part, norm2_dev, g.counter, live, gs);
+        launch_after((size_t)n * ncols * sizeof(C<T>), k_update_norm_c2, g.nblocks, kThreads, 0, s,
+                     reinterpret_cast<const float4 *>(V), ncols, dots_dev, reinterpret_cast<float4 *>(w), n / 2, part,
+                     norm2_dev, g.counter, live, gs);
     else
-        launch_after((size_t)n * ncols * sizeof(C<T>), k_update_norm<T>, g.nblocks, kThreads, 0, s, V, ncols, dots_dev, w, n, part, norm2_dev, g.counter,
-                     live, gs);
+        launch_after((size_t)n * ncols * sizeof(C<T>), k_update_norm<T>, g.nblocks, kThreads, 0, s, V, ncols, dots_dev,
+                     w, n, part, norm2_dev, g.counter, live, gs);
 }
 template <typename T>
 void VecOps<T>::update_norm(const C<T> *V, int ncols, const double2 *dots_dev, C<T> *w, long n, double *norm2_dev,

@@ -703,8 +703,8 @@ int egx_net_loss_grad(egx_ctx *ctx, egx_net *net, const float *v, const float *t
         EGX_CUDA(cudaMemsetAsync(e2, 0, 2 * batch * sizeof(double), s));
         k_loss_sums<<<dim3((unsigned)std::min<long>((per + 255) / 256, 512), batch), 256, 0, s>>>(
             net->Out.as<float>(), net->T.as<float>(), per, e2, t2);
-        k_loss_grad<<<dim3((unsigned)std::min<long>((per + 255) / 256, 1024), batch), 256, 0, s>>>(net->Out.as<float>(), net->T.as<float>(), t2, per, batch,
-                                                            net->dOut.as<float>());
+        k_loss_grad<<<dim3((unsigned)std::min<long>((per + 255) / 256, 1024), batch), 256, 0, s>>>(
+            net->Out.as<float>(), net->T.as<float>(), t2, per, batch, net->dOut.as<float>());
         ctx->launches += 3;
         backward(net, batch, s, &ctx->launches);
         std::vector<double> h(2 * batch);

@@ -244,7 +244,8 @@ static void launch_reg(int which, cudaStream_t s, int nlines, const C<T> *x, con
         launch_after(buffer_bytes<T>(*d), k_fwd_y_r<T, N, BT>, grid, thr, sm, s, x, *op, buf, *d, tw);
     } else if (which == 1) {
         reg_attr<T, N, BT>((const void *)k_lines_r<T, N, BT>);
-        launch_after((size_t)nlines * N * B * sizeof(C<T>), k_lines_r<T, N, BT>, grid, thr, sm, s, buf, lstride, estride, B, nload, nstore, tw, sign);
+        launch_after((size_t)nlines * N * B * sizeof(C<T>), k_lines_r<T, N, BT>, grid, thr, sm, s, buf, lstride,
+                     estride, B, nload, nstore, tw, sign);
     } else {
         reg_attr<T, N, BT>((const void *)k_bwd_y_r<T, N, BT>);
         launch_after(buffer_bytes<T>(*d), k_bwd_y_r<T, N, BT>, grid, thr, sm, s, buf, x, *op, y, *d, tw);
@@ -367,9 +368,9 @@ __global__ void k_contract(C<T> *buf, const C<T> *__restrict__ G, const OpDims d
 // ---------------------------------------------------------------------------
 // The complex128 contraction in double-FP32 arithmetic: the mixed form's
 // refinement residual where the digit products do not take it (nz > 48). GB300
-// runs complex128 FMAs at 1/64 of the FP32 rate,
-// which makes the FP64 block product above compute-bound; here every
-// operand is a pair of floats hi + lo (47 significant bits) and every dot
+// runs complex128 FMAs at 1/64 of the FP32 rate, which makes the FP64 block
+// product above compute-bound; here every operand is a pair of floats hi + lo
+// (47 significant bits) and every dot
 // product runs as Dot2 (Ogita, Rump and Oishi, "Accurate sum and dot
 // product", SIAM J. Sci. Comput. 26 (2005), Algorithm 5.3): each product
 // made error-free with one FMA (TwoProduct), each sum with Knuth's TwoSum,

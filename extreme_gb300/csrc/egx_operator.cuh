@@ -106,7 +106,7 @@ template <typename T>
 void fft_lines_sym(C<T> *buf, int nlines, long lstride, long estride, int B, int parity, int nstore, const FftPlan &p,
                    const C<T> *tw, int sign, cudaStream_t s, long *launches);
 
-// The generic transform's passes (egx_fft_gen.cu); false, and nothing
+// The generic transform's passes (egx_fft_gen_kernels.cuh); false, and nothing
 // launched, where the length has no such plan.
 template <typename T>
 bool gen_fwd_y(const FftPlan &p, const C<T> *x, const OperatorData<T> &op, C<T> *buf, const OpDims &d, const C<T> *tw,

@@ -262,7 +262,8 @@ class Context:
         self._check(self.lib.egx_op_apply(self.h, C.c_void_p(x_ptr), C.c_void_p(y_ptr), nrhs, DEVICE))
 
     def op_apply_ds(self, x, nrhs=1):
-        """Host arrays (complex128); the contraction in double-FP32."""
+        """Host arrays (complex128): the mixed form's residual apply
+        (egx_op_apply_ds)."""
         x = _c128(x)
         y = np.empty_like(x)
         self._check(self.lib.egx_op_apply_ds(self.h, _ptr(x), _ptr(y), nrhs, HOST))

@@ -179,7 +179,11 @@ int egx_op_prepare(egx_ctx *ctx, egx_green *g, const double *zeta, const double 
                    const double *dz, int type);
 /* Apply (ConvolutionOperator.cs:45-62,162-327): y = K x for nrhs vectors. */
 int egx_op_apply(egx_ctx *ctx, const double *x, double *y, int nrhs, int where);
-/* Same in complex64 (interleaved floats) with the complex64 tensor. */
+/* Same in complex64 (interleaved floats) with the complex64 tensor. FP32
+ * accuracy of every layer by itself, but for the sub-block layout of nz in
+ * {16, 32, 48}: there a tensor entry has 22 bits down to 2^-16 of the tensor's
+ * largest and none below 2^-38, and so has an entry of x beside the largest of
+ * its spectral column where two vectors are applied together (nrhs >= 2). */
 int egx_op_apply_c64(egx_ctx *ctx, const float *x, float *y, int nrhs, int where);
 /* The apply the mixed form uses for its refinement residuals: a complex128
  * apply whose block contraction needs no complex128 FMA. For nz <= 48 it is
